@@ -11,7 +11,8 @@
 // rows - the gate and the up tile of 128 h columns, or two neighbouring 128-feature tiles of the down
 // projection (256 contiguous bytes of every weight row) - so one K block is 2 x (128 x 32) accumulators, tensor
 // memory holds a ring of eight K blocks and the fold is 64 FMAs per thread per K block with the same
-// arithmetic as the large-batch kernel: acc += partial * (a_inv[row,kb] * w_inv[kb,nb]).
+// arithmetic as the large-batch kernel: acc += partial * (a_inv[row,kb] * w_inv[kb,nb]).  Of the 32 token columns only
+// the first 8 or 16 are read back and folded when the tile has no more rows than that (a batch of one: 8).
 // Same roles as there (reference: src/blackwell_moe/runtime/qwen_patch.py:108-129 computes these products
 // in bf16 after dequantising).
 //
@@ -20,6 +21,8 @@
 // (expert, 32 of its rows, 128 output features); tiles run expert-major, then feature block, then row block.
 // Every wait is bounded as in the other GEMM kernels; the fold warps meet on an mbarrier, not on bar.sync,
 // so that a warp that gave up cannot strand the others.
+#include <type_traits>
+
 #include "sm100_gemm.cuh"
 
 namespace bwmoe {
@@ -70,6 +73,9 @@ struct SmallCursor {
   }
 };
 
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8(taddr, r); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 __device__ __forceinline__ uint8_t e4m3_of(float v) {
   uint16_t r;
@@ -225,88 +231,92 @@ block_gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
       if (!cur.locate(tile, e, row0, row_end, ft)) break;
       const int n_valid = min(S_NT, row_end - row0);
       const uint32_t par = local & 1u;
-      // activation scales of the tile's rows: [K block][column]; rows past the segment take the first row's
-      for (int i = fold_tid; i < S_NT * k_blocks; i += 128) {
-        const int c = i / k_blocks, kb = i - c * k_blocks;
-        s_xinv[par][kb][c] = p.a_inv[(size_t)(row0 + (c < n_valid ? c : 0)) * k_blocks + kb];
-      }
-      // weight scales of the tile: lane kb holds K block kb's
-      float w0_reg, w1_reg;
-      {
-        const size_t at = ((size_t)e * k_blocks + min(lane, k_blocks - 1)) * p.nb;
-        if (GATE_UP) {
-          w0_reg = p.w0_inv[at + min(ft, p.nb - 1)];
-          w1_reg = p.w1_inv[at + min(ft, p.nb - 1)];
+      auto fold_tile = [&](auto columns) -> bool {
+        constexpr int NC = decltype(columns)::value;             // token columns that are read back
+        // activation scales of the tile's rows: [K block][column]; rows past the segment take the first row's
+        for (int i = fold_tid; i < NC * k_blocks; i += 128) {
+          const int c = i / k_blocks, kb = i - c * k_blocks;
+          s_xinv[par][kb][c] = p.a_inv[(size_t)(row0 + (c < n_valid ? c : 0)) * k_blocks + kb];
+        }
+        // weight scales of the tile: lane kb holds K block kb's
+        float w0_reg, w1_reg;
+        {
+          const size_t at = ((size_t)e * k_blocks + min(lane, k_blocks - 1)) * p.nb;
+          if (GATE_UP) {
+            w0_reg = p.w0_inv[at + min(ft, p.nb - 1)];
+            w1_reg = p.w1_inv[at + min(ft, p.nb - 1)];
+          } else {
+            w0_reg = p.w0_inv[at + min(2 * ft, p.nb - 1)];
+            w1_reg = p.w0_inv[at + min(2 * ft + 1, p.nb - 1)];
+          }
+        }
+        if (!fold_sync()) return false;
+        float acc0[NC], acc1[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc0[c] = 0.f, acc1[c] = 0.f;
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const uint32_t buf = it % S_NBUF, use = it / S_NBUF;
+          const float w0 = __shfl_sync(0xffffffffu, w0_reg, kb);
+          const float w1 = __shfl_sync(0xffffffffu, w1_reg, kb);
+          if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * buf, use & 1u, abort_flag, p.status))) return false;
+          tc_fence_after();
+          const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * S_BUF_COLS;
+          uint32_t r0[NC], r1[NC];
+          tmem_ld_cols(t_row, r0);
+          tmem_ld_cols(t_row + S_NT, r1);
+          tmem_ld_wait();
+          if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);      // the loads have landed: the buffer may be reused
+          const float* xs = s_xinv[par][kb];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const float a = xs[c];
+            acc0[c] = fmaf(__uint_as_float(r0[c]), a * w0, acc0[c]);
+            acc1[c] = fmaf(__uint_as_float(r1[c]), a * w1, acc1[c]);
+          }
+        }
+        const int n0 = ft * FT_COLS;
+        const bool f_ok = n0 + f_in_tile < p.N_out;
+        if constexpr (GATE_UP) {
+          // h = silu(gate) * up with the recipe's bf16 rounding points; one quantisation group = this tile's
+          // 128 features of a token, so the group maximum is a maximum over the 128 lanes of the four warps
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const float g = bf16r(acc0[c]), u = bf16r(acc1[c]);
+            const float a = bf16r(silu_f(g));
+            const float h = f_ok ? bf16r(a * u) : 0.f;
+            acc0[c] = h;
+            const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(h)));   // |h| >= 0: bit order = value order
+            if (lane == 0) s_cmax[par][quarter][c] = __uint_as_float(m);
+          }
+          if (!fold_sync()) return false;
+          uint8_t* out = static_cast<uint8_t*>(p.out);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            float amax = fmaxf(fmaxf(s_cmax[par][0][c], s_cmax[par][1][c]), fmaxf(s_cmax[par][2][c], s_cmax[par][3][c]));
+            amax = fmaxf(amax, kSmallAmaxFloor);
+            const float s = __fmul_rn(__frcp_rn(amax), kFp8Max);   // torch evaluates 448 / amax this way
+            if (c < n_valid) {
+              if (f_ok) out[(size_t)(row0 + c) * p.N_out + n0 + f_in_tile] = e4m3_of(acc0[c] * s);
+              if (f_in_tile == c) p.out_inv[(size_t)(row0 + c) * p.nb + ft] = __fdiv_rn(amax, kFp8Max);
+            }
+          }
         } else {
-          w0_reg = p.w0_inv[at + min(2 * ft, p.nb - 1)];
-          w1_reg = p.w0_inv[at + min(2 * ft + 1, p.nb - 1)];
-        }
-      }
-      if (!(ok = fold_sync())) break;
-      float acc0[S_NT], acc1[S_NT];
+          __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
+          const bool f1_ok = n0 + BN_HALF + f_in_tile < p.N_out;
 #pragma unroll
-      for (int c = 0; c < S_NT; ++c) acc0[c] = 0.f, acc1[c] = 0.f;
-      for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-        const uint32_t buf = it % S_NBUF, use = it / S_NBUF;
-        const float w0 = __shfl_sync(0xffffffffu, w0_reg, kb);
-        const float w1 = __shfl_sync(0xffffffffu, w1_reg, kb);
-        ok = mbar_wait(bar_tfull + 8 * buf, use & 1u, abort_flag, p.status);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * S_BUF_COLS;
-        uint32_t r0[32], r1[32];
-        tmem_ld32(t_row, r0);
-        tmem_ld32(t_row + S_NT, r1);
-        tmem_ld_wait();
-        if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);      // the loads have landed: the buffer may be reused
-        const float* xs = s_xinv[par][kb];
-#pragma unroll
-        for (int c = 0; c < S_NT; ++c) {
-          const float a = xs[c];
-          acc0[c] = fmaf(__uint_as_float(r0[c]), a * w0, acc0[c]);
-          acc1[c] = fmaf(__uint_as_float(r1[c]), a * w1, acc1[c]);
-        }
-      }
-      if (!ok) break;
-      const int n0 = ft * FT_COLS;
-      const bool f_ok = n0 + f_in_tile < p.N_out;
-      if constexpr (GATE_UP) {
-        // h = silu(gate) * up with the recipe's bf16 rounding points; one quantisation group = this tile's
-        // 128 features of a token, so the group maximum is a maximum over the 128 lanes of the four warps
-#pragma unroll
-        for (int c = 0; c < S_NT; ++c) {
-          const float g = bf16r(acc0[c]), u = bf16r(acc1[c]);
-          const float a = bf16r(silu_f(g));
-          const float h = f_ok ? bf16r(a * u) : 0.f;
-          acc0[c] = h;
-          const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(h)));   // |h| >= 0: bit order = value order
-          if (lane == 0) s_cmax[par][quarter][c] = __uint_as_float(m);
-        }
-        if (!(ok = fold_sync())) break;
-        uint8_t* out = static_cast<uint8_t*>(p.out);
-#pragma unroll
-        for (int c = 0; c < S_NT; ++c) {
-          float amax = fmaxf(fmaxf(s_cmax[par][0][c], s_cmax[par][1][c]), fmaxf(s_cmax[par][2][c], s_cmax[par][3][c]));
-          amax = fmaxf(amax, kSmallAmaxFloor);
-          const float s = __fmul_rn(__frcp_rn(amax), kFp8Max);   // torch evaluates 448 / amax this way
-          if (c < n_valid) {
-            if (f_ok) out[(size_t)(row0 + c) * p.N_out + n0 + f_in_tile] = e4m3_of(acc0[c] * s);
-            if (f_in_tile == c) p.out_inv[(size_t)(row0 + c) * p.nb + ft] = __fdiv_rn(amax, kFp8Max);
+          for (int c = 0; c < NC; ++c) {
+            if (c < n_valid) {
+              __nv_bfloat16* row = out + (size_t)(row0 + c) * p.N_out + n0 + f_in_tile;
+              if (f_ok) row[0] = __float2bfloat16_rn(acc0[c]);
+              if (f1_ok) row[BN_HALF] = __float2bfloat16_rn(acc1[c]);
+            }
           }
         }
-      } else {
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
-        const bool f1_ok = n0 + BN_HALF + f_in_tile < p.N_out;
-#pragma unroll
-        for (int c = 0; c < S_NT; ++c) {
-          if (c < n_valid) {
-            __nv_bfloat16* row = out + (size_t)(row0 + c) * p.N_out + n0 + f_in_tile;
-            if (f_ok) row[0] = __float2bfloat16_rn(acc0[c]);
-            if (f1_ok) row[BN_HALF] = __float2bfloat16_rn(acc1[c]);
-          }
-        }
-      }
+        return true;
+      };
+      ok = n_valid <= 8    ? fold_tile(std::integral_constant<int, 8>{})
+           : n_valid <= 16 ? fold_tile(std::integral_constant<int, 16>{})
+                           : fold_tile(std::integral_constant<int, S_NT>{});
     }
   }
 
