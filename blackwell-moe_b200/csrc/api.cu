@@ -215,26 +215,27 @@ int run_pipeline(const void* x, const float* weights, const int32_t* indices, co
   float* amax_h = at<float>(ws, L.amax_h);
   float* scale_x = at<float>(ws, L.scale_x);
   float* scale_h = at<float>(ws, L.scale_h);
-  int rc;
-  if ((rc = launch_plan(indices, row_amax, T, E, K, offsets, pos, row_slot, row_expert, amax_x, status,
-                        at<void>(ws, L.plan_scratch), st, scale_x)))
-    return rc;
   float* row_w = at<float>(ws, L.row_w);
-  if ((rc = launch_scatter_quant(x, pos, indices, scale_x, T, D, K, at<void>(ws, L.xq), st, weights, row_w))) return rc;
+  int rc;
+  if (plan_quant_applicable(T, E, K)) {       // decode-sized batches: plan and quantisation in one launch
+    if ((rc = launch_plan_quant(x, indices, row_amax, weights, T, D, E, K, offsets, pos, row_slot, row_expert, amax_x, scale_x,
+                                status, at<void>(ws, L.xq), row_w, nullptr, st)))
+      return rc;
+  } else {
+    if ((rc = launch_plan(indices, row_amax, T, E, K, offsets, pos, row_slot, row_expert, amax_x, status,
+                          at<void>(ws, L.plan_scratch), st, scale_x)))
+      return rc;
+    if ((rc = launch_scatter_quant(x, pos, indices, scale_x, T, D, K, at<void>(ws, L.xq), st, weights, row_w))) return rc;
+  }
   const FusedRequant fr{at<void>(ws, L.hq), scale_h, at<unsigned int>(ws, L.arrivals)};
   bool requant_done = false;
-  // The always-on groups E-n_shared .. E-1 are column pieces of ONE shared MLP whose h is quantised with one
-  // scale (FP8SharedExpert, shared_expert_fp8.py:64): their maxima are merged before the requantisation,
-  // which therefore cannot be fused into the small-batch SwiGLU kernel.
-  const bool merge = n_shared > 1;
   if ((rc = launch_gateup(at<void>(ws, L.xq), offsets, scale_x, wg, wu, sg, su, M, D, H, E, at<void>(ws, L.h),
-                          amax_h, status, at<void>(ws, L.gemm_scratch), st, merge ? nullptr : &fr,
-                          merge ? nullptr : &requant_done)))
+                          amax_h, status, at<void>(ws, L.gemm_scratch), st, &fr, &requant_done, n_shared)))
     return rc;
-  if (merge && (rc = launch_merge_amax(amax_h, E - n_shared, n_shared, st))) return rc;
   // scale_h is derived from amax_h inside the requantisation kernel
   if (!requant_done &&
-      (rc = launch_requant(at<void>(ws, L.h), row_expert, amax_h, M, H, at<void>(ws, L.hq), st, scale_h)))
+      (rc = launch_requant(at<void>(ws, L.h), row_expert, amax_h, M, H, at<void>(ws, L.hq), st, scale_h,
+                           n_shared > 0 ? E - n_shared : E - 1)))
     return rc;
   CombineArgs ca{pos, weights, T, K, out, out_scale, residual};
   ca.row_w = row_w;
@@ -262,16 +263,6 @@ __global__ void row_amax_kernel(const __nv_bfloat16* __restrict__ x, int T, int 
   if (lane == 0) row_amax[t] = m;
 }
 
-// Expert ids of the whole model -> slots of a resident expert pool.  An id outside [0, n_ids) or an
-// expert without a slot (remap < 0) becomes -1, which the plan reports as BWMOE_STATUS_BAD_EXPERT.
-__global__ void remap_ids_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ remap, int n_ids,
-                                 int n, int32_t* __restrict__ slots) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int id = ids[i];
-  slots[i] = (id >= 0 && id < n_ids) ? remap[id] : -1;
-}
-
 // The block-scale pipeline behind the routing: plan -> per-token group quantisation -> rows into expert
 // order -> gate/up (+ SwiGLU + requant) -> down -> combine.
 int run_block_pipeline(const void* x, const float* weights, const int32_t* indices, const void* wg, const void* wu,
@@ -281,12 +272,19 @@ int run_block_pipeline(const void* x, const float* weights, const int32_t* indic
   int32_t* status = at<int32_t>(ws, L.status);
   int32_t* offsets = at<int32_t>(ws, L.offsets);
   int rc;
-  if ((rc = launch_plan(indices, nullptr, T, E, K, offsets, at<int32_t>(ws, L.pos), at<int32_t>(ws, L.row_slot),
-                        at<int32_t>(ws, L.row_expert), nullptr, status, at<void>(ws, L.plan_scratch), st)))
-    return rc;
-  // token-major: a row is read and quantised once, its codes and group scales written to its K rows
-  if ((rc = launch_quant_scatter_group(x, at<int32_t>(ws, L.pos), T, D, K, at<void>(ws, L.xq), at<float>(ws, L.x_inv), st)))
-    return rc;
+  if (plan_quant_applicable(T, E, K)) {       // plan and quantisation in one launch, as in run_pipeline
+    if ((rc = launch_plan_quant(x, indices, nullptr, weights, T, D, E, K, offsets, at<int32_t>(ws, L.pos),
+                                at<int32_t>(ws, L.row_slot), at<int32_t>(ws, L.row_expert), nullptr, nullptr, status,
+                                at<void>(ws, L.xq), nullptr, at<float>(ws, L.x_inv), st)))
+      return rc;
+  } else {
+    if ((rc = launch_plan(indices, nullptr, T, E, K, offsets, at<int32_t>(ws, L.pos), at<int32_t>(ws, L.row_slot),
+                          at<int32_t>(ws, L.row_expert), nullptr, status, at<void>(ws, L.plan_scratch), st)))
+      return rc;
+    // token-major: a row is read and quantised once, its codes and group scales written to its K rows
+    if ((rc = launch_quant_scatter_group(x, at<int32_t>(ws, L.pos), T, D, K, at<void>(ws, L.xq), at<float>(ws, L.x_inv), st)))
+      return rc;
+  }
   if ((rc = launch_gateup_block(at<void>(ws, L.xq), at<float>(ws, L.x_inv), offsets, wg, wu, inv_g, inv_u, M, D, H, E,
                                 at<void>(ws, L.hq), at<float>(ws, L.h_inv), status, st)))
     return rc;
@@ -428,12 +426,11 @@ int bwmoe_moe_forward(const void* x, const void* w_gate, const void* wg, const v
     return rc;
   BWMOE_REQUIRE(w_gate != nullptr, BWMOE_ERR_NULL, "moe_forward: w_gate is null");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   float* weights = at<float>(ws, L.topk_w);
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status)))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st);
 }
@@ -447,12 +444,11 @@ int bwmoe_moe_forward_flags(const void* x, const void* w_gate, const void* wg, c
   BWMOE_REQUIRE(w_gate != nullptr, BWMOE_ERR_NULL, "moe_forward_flags: w_gate is null");
   BWMOE_REQUIRE((flags & ~BWMOE_FLAG_REDUCE_COMBINE) == 0, BWMOE_ERR_UNSUPPORTED, "moe_forward_flags: unknown flag bits %#x", flags);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   float* weights = at<float>(ws, L.topk_w);
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status)))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st, 1.0f, nullptr,
                       flags);
@@ -469,18 +465,13 @@ int bwmoe_moe_forward_shared(const void* x, const void* w_gate, const void* wg, 
     return rc;
   BWMOE_REQUIRE(w_gate != nullptr, BWMOE_ERR_NULL, "moe_forward_shared: w_gate is null");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
-  // routing of the E routed experts into scratch that later stages overwrite (pos, row_w), then the S always-on
-  // slots are appended: indices / weights [T, K+S]
-  int32_t* idx_r = at<int32_t>(ws, L.pos);
-  float* w_r = at<float>(ws, L.row_w);
+  // routing of the E routed experts; the router appends the S always-on slots: indices / weights [T, K+S]
   float* weights = at<float>(ws, L.topk_w);
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
-  if (int rc = launch_router(x, w_gate, T, D, E, K, w_r, idx_r, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status)))
+  if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, S, ws, L.zero_end))
     return rc;
-  if (int rc = launch_append_shared_slots(idx_r, w_r, T, K, E, S, indices, weights, st)) return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E + S, K + S, out, ws, L, st,
                       routed_scale, nullptr, 0, S);
 }
@@ -495,12 +486,11 @@ int bwmoe_moe_forward_ex(const void* x, const void* w_gate, const void* wg, cons
   BWMOE_REQUIRE(w_gate != nullptr, BWMOE_ERR_NULL, "moe_forward_ex: w_gate is null");
   BWMOE_REQUIRE(residual == nullptr || aligned16(residual), BWMOE_ERR_BAD_ALIGN, "moe_forward_ex: residual alignment");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   float* weights = at<float>(ws, L.topk_w);
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status)))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st,
                       routed_scale, residual);
@@ -549,15 +539,11 @@ int bwmoe_moe_forward_routed(const void* x, const float* weights, const int32_t*
     return rc;
   BWMOE_REQUIRE(weights && indices, BWMOE_ERR_NULL, "moe_forward_routed: routing is null");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   float* row_amax = at<float>(ws, L.row_amax);
-  row_amax_kernel<<<ceil_div(T, 8), 256, 0, counted(st)>>>(static_cast<const __nv_bfloat16*>(x), T, D, row_amax);
-  BWMOE_CUDA_OK(cudaGetLastError());
-  // keep a copy of the routing in the workspace so that the views stay meaningful
-  BWMOE_CUDA_OK(cudaMemcpyAsync(at<void>(ws, L.topk_idx), indices, sizeof(int32_t) * (size_t)T * K,
-                                cudaMemcpyDeviceToDevice, st));
-  BWMOE_CUDA_OK(cudaMemcpyAsync(at<void>(ws, L.topk_w), weights, sizeof(float) * (size_t)T * K,
-                                cudaMemcpyDeviceToDevice, st));
+  // keeps a copy of the routing in the workspace so that the views stay meaningful
+  if (int rc = launch_routed_prepare(x, weights, indices, nullptr, 0, T, D, K, at<float>(ws, L.topk_w),
+                                     at<int32_t>(ws, L.topk_idx), row_amax, ws, L.zero_end, st))
+    return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st);
 }
 
@@ -572,16 +558,11 @@ int bwmoe_moe_forward_routed_remap(const void* x, const float* weights, const in
   BWMOE_REQUIRE(weights && expert_ids && remap, BWMOE_ERR_NULL, "moe_forward_routed_remap: routing or remap is null");
   BWMOE_REQUIRE(n_experts_total > 0, BWMOE_ERR_BAD_SHAPE, "moe_forward_routed_remap: %d experts", n_experts_total);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int M = T * K;
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   float* row_amax = at<float>(ws, L.row_amax);
-  row_amax_kernel<<<ceil_div(T, 8), 256, 0, counted(st)>>>(static_cast<const __nv_bfloat16*>(x), T, D, row_amax);
-  BWMOE_CUDA_OK(cudaGetLastError());
   int32_t* slots = at<int32_t>(ws, L.topk_idx);                 // the workspace's routing view holds slot ids
-  remap_ids_kernel<<<ceil_div(M, 256), 256, 0, counted(st)>>>(expert_ids, remap, n_experts_total, M, slots);
-  BWMOE_CUDA_OK(cudaGetLastError());
-  BWMOE_CUDA_OK(cudaMemcpyAsync(at<void>(ws, L.topk_w), weights, sizeof(float) * (size_t)M,
-                                cudaMemcpyDeviceToDevice, st));
+  if (int rc = launch_routed_prepare(x, weights, expert_ids, remap, n_experts_total, T, D, K, at<float>(ws, L.topk_w), slots,
+                                     row_amax, ws, L.zero_end, st))
+    return rc;
   return run_pipeline(x, weights, slots, row_amax, wg, wu, wd, sg, su, sd, T, D, H, n_slots, K, out, ws, L, st);
 }
 
@@ -647,11 +628,10 @@ int bwmoe_moe_forward_block(const void* x, const void* w_gate, const void* wg, c
     return rc;
   BWMOE_REQUIRE(w_gate != nullptr, BWMOE_ERR_NULL, "moe_forward_block: w_gate is null");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   float* weights = at<float>(ws, L.topk_w);
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, nullptr, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status)))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
     return rc;
   return run_block_pipeline(x, weights, indices, wg, wu, wd, inv_g, inv_u, inv_d, T, D, H, E, K, out, ws, L, st);
 }
@@ -669,17 +649,10 @@ int bwmoe_moe_forward_block_routed(const void* x, const float* weights, const in
   BWMOE_REQUIRE(remap == nullptr || n_experts_total > 0, BWMOE_ERR_BAD_SHAPE,
                 "moe_forward_block_routed: remap given with %d experts", n_experts_total);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int M = T * K;
-  BWMOE_CUDA_OK(cudaMemsetAsync(ws, 0, L.zero_end, st));
   int32_t* slots = at<int32_t>(ws, L.topk_idx);
-  if (remap != nullptr) {
-    remap_ids_kernel<<<ceil_div(M, 256), 256, 0, counted(st)>>>(expert_ids, remap, n_experts_total, M, slots);
-    BWMOE_CUDA_OK(cudaGetLastError());
-  } else {
-    BWMOE_CUDA_OK(cudaMemcpyAsync(slots, expert_ids, sizeof(int32_t) * (size_t)M, cudaMemcpyDeviceToDevice, st));
-  }
-  BWMOE_CUDA_OK(cudaMemcpyAsync(at<void>(ws, L.topk_w), weights, sizeof(float) * (size_t)M,
-                                cudaMemcpyDeviceToDevice, st));
+  if (int rc = launch_routed_prepare(x, weights, expert_ids, remap, n_experts_total, T, D, K, at<float>(ws, L.topk_w), slots,
+                                     nullptr, ws, L.zero_end, st))
+    return rc;
   return run_block_pipeline(x, weights, slots, wg, wu, wd, inv_g, inv_u, inv_d, T, D, H, n_slots, K, out, ws, L, st);
 }
 

@@ -84,6 +84,7 @@ constexpr float kFp8Max = 448.0f;
 // The reference clamps amax in the tensor's own dtype (bf16), so the floor is
 // bf16(1e-4) = 0x38D2, not the fp32 literal.
 constexpr float kAmaxFloor = 0.00010013580322265625f;
+constexpr float kGroupAmaxFloor = 1e-4f;      // of a 128-element group of the block-scale recipe (an fp32 maximum)
 
 // The reference writes `448.0 / amax` with a Python scalar on the left, which torch
 // evaluates as reciprocal(amax) * 448 (two roundings); reproduce exactly that.
@@ -109,25 +110,48 @@ __device__ __forceinline__ void atomic_max_nonneg(float* addr, float v) {
   atomicMax(reinterpret_cast<unsigned int*>(addr), __float_as_uint(v));
 }
 
+// Where a router kernel writes its result: token t's K routed slots at row t of [T, ld] arrays, followed by n_tail
+// always-on slots - experts E .. E+n_tail-1, which the router does not score, each with weight 1.
+struct RouteRows {
+  float* weights;
+  int32_t* indices;
+  int ld, n_tail;
+  __device__ __forceinline__ void write_tail(size_t tok, int lane, int E, int K) const {
+    if (lane < n_tail) {
+      weights[tok * ld + K + lane] = 1.0f;
+      indices[tok * ld + K + lane] = E + lane;
+    }
+  }
+};
+
 // ---- launchers implemented in the individual .cu files ---------------------
 // scratch (optional): enables the tensor-core router where it applies; needs router_scratch_bytes()
+// n_tail: always-on slots appended to every token's K (see RouteRows; weights / indices are [T, K + n_tail]).
+// zero: words to be cleared before any later kernel of the stream runs (and before `status` can be raised).
 // T_as > 0: choose the routing kernel a batch of T_as tokens would get (the kernels agree on the selected
 // experts always, but their fp32 weights differ in the last bits: a rank that routes a slice of a larger batch
 // passes the size of the whole batch to obtain the weights the whole batch would have got).
 size_t router_scratch_bytes(int T, int D, int E, int K, int T_as = 0);
 int launch_router(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
                   int32_t* indices, float* row_amax, cudaStream_t st, void* scratch = nullptr,
-                  size_t scratch_bytes = 0, int32_t* status = nullptr, int T_as = 0);
+                  size_t scratch_bytes = 0, int32_t* status = nullptr, int T_as = 0, int n_tail = 0,
+                  void* zero = nullptr, size_t zero_bytes = 0);
 bool router_tc_applicable(int T, int D, int E, int K);
 size_t router_tc_scratch_bytes(int T, int D, int E);
-int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, float* weights, int32_t* indices,
+int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
                      float* row_amax, int32_t* status, void* scratch, cudaStream_t st);
-int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
-                           int32_t* indices, const int32_t* list, const int32_t* count, cudaStream_t st);
+int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
+                           const int32_t* list, const int32_t* count, cudaStream_t st);
 size_t plan_scratch_bytes(int T, int E, int K);
 int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                 int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,
                 void* scratch, cudaStream_t st, float* scales_out = nullptr);
+// Plan and quantisation of a decode-sized batch in one launch (x_inv != nullptr: the block-scale recipe).  Only inside
+// the whole-block forwards: x is read before the kernel in front of it has finished.
+bool plan_quant_applicable(int T, int E, int K);
+int launch_plan_quant(const void* x, const int32_t* indices, const float* row_amax, const float* weights, int T, int D, int E,
+                      int K, int32_t* offsets, int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax,
+                      float* scales, int32_t* status, void* xq, float* row_w, float* x_inv, cudaStream_t st);
 int launch_plan_static(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                        int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,
                        cudaStream_t st);
@@ -147,19 +171,22 @@ int launch_combine_peers(void* const* src, int n_ranks, const int32_t* pos, cons
 int launch_gather_quant(const void* x, const int32_t* row_slot, const int32_t* row_expert,
                         const float* scales, int M, int D, int K, void* xq, cudaStream_t st);
 int launch_requant(const void* h, const int32_t* row_expert, const float* scales_h, int M, int H,
-                   void* hq, cudaStream_t st, float* scales_from_amax_out = nullptr);
+                   void* hq, cudaStream_t st, float* scales_from_amax_out = nullptr, int amax_last = 255);
 int launch_requant_segments(const void* h, const int32_t* offsets, const float* scales_h, int E, int H, void* hq,
                             cudaStream_t st);
 int launch_combine(const void* y, const int32_t* pos, const float* weights, int T, int D, int K,
                    void* out, cudaStream_t st, float scale = 1.0f, const void* residual = nullptr,
                    bool preweighted = false, int n_tail = 0);
-int launch_append_shared_slots(const int32_t* idx_r, const float* w_r, int T, int K, int E, int S, int32_t* idx,
-                               float* w, cudaStream_t st);
-int launch_merge_amax(float* amax, int first, int count, cudaStream_t st);
+int launch_routed_prepare(const void* x, const float* weights, const int32_t* ids, const int32_t* remap, int n_ids, int T,
+                          int D, int K, float* w_out, int32_t* slots, float* row_amax, void* zero, size_t zero_bytes,
+                          cudaStream_t st);
 int launch_dense_prepare(const float* row_amax, int T, int32_t* offsets, float* seg_amax, cudaStream_t st);
 int launch_quant_rows_from_amax(const void* x, const int32_t* row_expert, const float* seg_amax, int M, int W,
                                 void* xq, float* scales_out, cudaStream_t st);
 size_t gemm_scratch_bytes(int M, int D, int H, int E);
+// n_tail of launch_gateup: the last n_tail groups are column pieces of ONE always-on MLP whose h is quantised with one
+// scale (FP8SharedExpert, src/blackwell_moe/runtime/shared_expert_fp8.py:64): they share the entry of the first of
+// them in amax_h.  launch_requant finds it through amax_last, the last entry that is in use.
 // Handed to launch_gateup by the whole-forward entry points: where the requantised h, its scales and the
 // zero-initialised arrival counter of the fused small-batch kernel live.  *requant_done tells the caller
 // whether hq and scale_h were produced (then no 16-bit h exists and no requantisation pass is needed).
@@ -171,7 +198,7 @@ struct FusedRequant {
 int launch_gateup(const void* xq, const int32_t* offsets, const float* sx, const void* wg, const void* wu,
                   const float* sg, const float* su, int M, int D, int H, int E, void* h, float* amax_h,
                   int32_t* status, void* scratch, cudaStream_t st, const FusedRequant* fr = nullptr,
-                  bool* requant_done = nullptr);
+                  bool* requant_done = nullptr, int n_tail = 0);
 // What the weighted combine needs; handed to launch_down so that a split-K down projection can sum its
 // slabs and combine in one kernel (*fused reports whether it did; otherwise the caller combines).
 struct CombineArgs {

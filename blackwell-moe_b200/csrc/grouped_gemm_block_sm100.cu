@@ -38,7 +38,6 @@ constexpr int FOLD_WARP0 = 4;             // first fold warp
 constexpr int REGS_SMALL = 40;            // per thread after setmaxnreg: first warpgroup
 constexpr int REGS_FOLD = 232;            //                              fold warpgroups  (128*40 + 256*232 = 384*168)
 constexpr int SCALE_KB_MAX = 16;          // K blocks whose activation scales the shared-memory staging holds
-constexpr float kGroupAmaxFloor = 1e-4f;
 
 __device__ __forceinline__ void cp_async4(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst_smem), "l"(src) : "memory");

@@ -65,6 +65,7 @@ struct GemmParams {
   const int32_t* row_slot = nullptr;
   void* tok_out = nullptr;
   int top_k = 1;
+  int amax_last = 255;  // GATE_UP: segments from this one on share its entry of seg_amax
 };
 
 
@@ -363,7 +364,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // (zero-filled columns give h = 0, which cannot raise the maximum)
         if (!row_ok) amax = 0.f;
         for (int off = 16; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-        if (lane == 0 && amax > 0.f) atomic_max_nonneg(p.seg_amax + e, amax);
+        if (lane == 0 && amax > 0.f) atomic_max_nonneg(p.seg_amax + min(e, p.amax_last), amax);
       } else {
         const float sa = p.scale_a[e];
         const float inv = 1.0f / (sa * p.scale_b0[e]);
@@ -467,7 +468,8 @@ __device__ __forceinline__ int expert_of_row(const int32_t* __restrict__ offsets
 __global__ void __launch_bounds__(256)
 swiglu_from_partials_kernel(const float* __restrict__ partial, int S, int M, int H, const int32_t* __restrict__ offsets,
                             int E, const float* __restrict__ sx, const float* __restrict__ sg,
-                            const float* __restrict__ su, __nv_bfloat16* __restrict__ h, float* __restrict__ seg_amax) {
+                            const float* __restrict__ su, __nv_bfloat16* __restrict__ h, float* __restrict__ seg_amax,
+                            int amax_last) {
   chain_wait();
   const int vec_per_row = H / 4;
   const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -504,14 +506,14 @@ swiglu_from_partials_kernel(const float* __restrict__ partial, int S, int M, int
         make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
   }
   // one atomic per warp when the whole warp works on one expert (the common case), else per thread
-  const int key = live ? e : -1;
+  const int key = live ? min(e, amax_last) : -1;
   const int key0 = __shfl_sync(0xffffffffu, key, 0);
   if (__all_sync(0xffffffffu, key == key0)) {
     float mx = amax;
     for (int off = 16; off; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     if ((threadIdx.x & 31) == 0 && key0 >= 0 && mx > 0.f) atomic_max_nonneg(seg_amax + key0, mx);
   } else if (live && amax > 0.f) {
-    atomic_max_nonneg(seg_amax + e, amax);
+    atomic_max_nonneg(seg_amax + key, amax);
   }
 }
 
@@ -528,7 +530,7 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
                                     const float* __restrict__ sg, const float* __restrict__ su,
                                     uint8_t* __restrict__ hq, float* __restrict__ seg_amax,
                                     float* __restrict__ scale_h, unsigned int* __restrict__ arrivals,
-                                    int32_t* __restrict__ status) {
+                                    int32_t* __restrict__ status, int amax_last) {
   chain_wait();
   __shared__ int s_ok;
   const int vec_per_row = H / 4;
@@ -570,7 +572,7 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
     }
     // one atomic per warp when the whole warp works on one expert (the common case), else per thread: tens of
     // thousands of atomics on one address would serialise for longer than the rest of the kernel takes
-    const int key = ex[i];
+    const int key = min(ex[i], amax_last);          // -1 stays -1
     const int key0 = __shfl_sync(0xffffffffu, key, 0);
     if (__all_sync(0xffffffffu, key == key0)) {
       float mx = amax;
@@ -612,7 +614,7 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
     if (ex[i] < 0) continue;
     const long long item = ((long long)i * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
     const int m = (int)(item / vec_per_row), v = (int)(item % vec_per_row);
-    const float scale = scale_from_amax(__ldcg(seg_amax + ex[i]));
+    const float scale = scale_from_amax(__ldcg(seg_amax + min(ex[i], amax_last)));
     if (v == 0) scale_h[ex[i]] = scale;            // every row of the segment writes the same value
     reinterpret_cast<uint32_t*>(hq + (size_t)m * H)[v] =
         (uint32_t)to_e4m3x2(hv[i][0] * scale, hv[i][1] * scale) |
@@ -799,7 +801,7 @@ size_t gemm_scratch_bytes(int M, int D, int H, int /*E*/) {
 
 int launch_gateup(const void* xq, const int32_t* offsets, const float* sx, const void* wg, const void* wu,
                   const float* sg, const float* su, int M, int D, int H, int E, void* h, float* amax_h,
-                  int32_t* status, void* scratch, cudaStream_t st, const FusedRequant* fr, bool* requant_done) {
+                  int32_t* status, void* scratch, cudaStream_t st, const FusedRequant* fr, bool* requant_done, int n_tail) {
   if (requant_done) *requant_done = false;
   BWMOE_REQUIRE(xq && offsets && sx && wg && wu && sg && su && h && amax_h && status, BWMOE_ERR_NULL,
                 "gateup: null pointer");
@@ -812,6 +814,7 @@ int launch_gateup(const void* xq, const int32_t* offsets, const float* sx, const
   const int k_blocks = ceil_div(D, BK), n_tiles = ceil_div(H, BN_HALF);
   const SplitPlan sp = choose_split(M, E, k_blocks, n_tiles);
   GemmParams p{offsets, sx, sg, su, h, amax_h, status, E, D, H, n_tiles, sp.split_k, sp.k_per_split, M, 2 * H, nullptr};
+  p.amax_last = n_tail > 0 ? E - n_tail : E - 1;
   if (sp.split_k == 1) return launch_gemm<true, false>(ma, mg, mu, p, M, st);
   BWMOE_REQUIRE(scratch != nullptr && aligned16(scratch), BWMOE_ERR_WORKSPACE, "gateup: scratch buffer required");
   p.partial = static_cast<float*>(scratch);
@@ -824,13 +827,13 @@ int launch_gateup(const void* xq, const int32_t* offsets, const float* sx, const
   if (fr != nullptr && requant_done != nullptr && n <= fused_blocks * 256 * kFusedItems) {
     BWMOE_CUDA_OK(launch_chained(swiglu_requant_from_partials_kernel, dim3((unsigned)fused_blocks), dim3(256), 0, st,
         p.partial, sp.split_k, M, H, offsets, E, sx, sg, su, static_cast<uint8_t*>(fr->hq), amax_h, fr->scale_h,
-        fr->arrivals, status));
+        fr->arrivals, status, p.amax_last));
     BWMOE_CUDA_OK(cudaGetLastError());
     *requant_done = true;
     return BWMOE_OK;
   }
   BWMOE_CUDA_OK(launch_chained(swiglu_from_partials_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st,
-      p.partial, sp.split_k, M, H, offsets, E, sx, sg, su, static_cast<__nv_bfloat16*>(h), amax_h));
+      p.partial, sp.split_k, M, H, offsets, E, sx, sg, su, static_cast<__nv_bfloat16*>(h), amax_h, p.amax_last));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }

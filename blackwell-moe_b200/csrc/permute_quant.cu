@@ -5,6 +5,7 @@
 // src/blackwell_moe/kernels/fp8_moe_v3.py:39-48, of the Triton segment kernels
 // (src/blackwell_moe/kernels/segment_ops.py:15-120) and of the scatter-add combine
 // (src/blackwell_moe/kernels/scatter.py:25-72).
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -131,66 +132,100 @@ plan_rank_kernel(const int32_t* __restrict__ indices, int M, int E, const int32_
 }
 
 // ---- all three passes in one block, for at most 1024 slots (decode-sized batches) ----
-// Also emits the per-segment quantisation scale when asked to (scales_out != nullptr).
+struct SmallPlan {
+  int start[kMaxE + 1];        // first row of each expert; [E] = rows that exist
+  unsigned int amax[kMaxE];    // bits of the segment's max|x|
+};
+// Called by all 1024 threads of a block; thread s owns slot s.  `cnt` is shared memory for 32 * (E + 1) ints.
+// Returns the slot's expert (-1: out of range or no slot) and its permuted row in `row`.  The two scans run on
+// shuffles - across the 32 warps for one expert per warp at a time, and over the experts in warp 0 - because a
+// thread that walks E running sums through shared memory takes longer (256 x ~30 cycles) than everything else here.
+__device__ int small_plan(const int32_t* __restrict__ indices, const float* __restrict__ row_amax, int M, int E, int K,
+                          int* cnt, SmallPlan& sp, int32_t* __restrict__ status, bool report, int& row) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = threadIdx.x, ld = E + 1;
+  int e = s < M ? indices[s] : -1;
+  const float am = (s < M && row_amax != nullptr) ? row_amax[s / K] : 0.f;
+  for (int i = threadIdx.x; i < 32 * ld; i += kPlanThreads) cnt[i] = 0;
+  for (int i = threadIdx.x; i < E; i += kPlanThreads) sp.amax[i] = 0u;
+  __syncthreads();
+  if (s < M && (e < 0 || e >= E)) {
+    if (report) atomicOr(status, BWMOE_STATUS_BAD_EXPERT);
+    e = -1;
+  }
+  if (e >= 0 && row_amax != nullptr) atomicMax(&sp.amax[e], __float_as_uint(am));
+  const unsigned peers = __match_any_sync(0xffffffffu, e);
+  const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
+  if (e >= 0 && rank_in_warp == 0) cnt[warp * ld + e] = __popc(peers);
+  __syncthreads();
+  for (int ee = warp; ee < E; ee += 32) {          // lane l: warp l's count of expert ee (the odd stride spreads the banks)
+    const int c = cnt[lane * ld + ee];
+    int incl = c;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+    cnt[lane * ld + ee] = incl - c;
+    if (lane == 31) sp.start[ee + 1] = incl;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int v[kMaxE / 32], run = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxE / 32; ++j) {
+      const int ee = lane * (kMaxE / 32) + j;
+      run += ee < E ? sp.start[ee + 1] : 0;
+      v[j] = run;
+    }
+    int incl = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+#pragma unroll
+    for (int j = 0; j < kMaxE / 32; ++j) {
+      const int ee = lane * (kMaxE / 32) + j;
+      if (ee < E) sp.start[ee + 1] = incl - run + v[j];
+    }
+    if (lane == 0) sp.start[0] = 0;
+  }
+  __syncthreads();
+  row = e >= 0 ? sp.start[e] + cnt[warp * ld + e] + rank_in_warp : -1;
+  return e;
+}
+// One block writes the plan: offsets, both directions of the permutation, segment amax and (optionally) scales.
+__device__ void publish_small_plan(const SmallPlan& sp, int M, int E, int e, int row, int32_t* __restrict__ offsets,
+                                   int32_t* __restrict__ pos, int32_t* __restrict__ row_slot,
+                                   int32_t* __restrict__ row_expert, float* __restrict__ seg_amax,
+                                   float* __restrict__ scales_out) {
+  const int s = threadIdx.x;
+  for (int ee = threadIdx.x; ee <= E; ee += kPlanThreads) offsets[ee] = sp.start[ee];
+  for (int ee = threadIdx.x; ee < E; ee += kPlanThreads) {
+    const float a = __uint_as_float(sp.amax[ee]);
+    if (seg_amax != nullptr) seg_amax[ee] = a;
+    if (scales_out != nullptr) scales_out[ee] = sp.start[ee + 1] > sp.start[ee] ? scale_from_amax(a) : 1.0f;
+  }
+  if (s < M) pos[s] = row;
+  if (e >= 0) {
+    row_slot[row] = s;
+    row_expert[row] = e;
+  }
+  // rows past the last segment (slots with an out-of-range expert id own none): marked as absent
+  if (s < M && s >= sp.start[E]) row_slot[s] = -1, row_expert[s] = -1;
+}
+
 __global__ void __launch_bounds__(kPlanThreads)
 plan_small_kernel(const int32_t* __restrict__ indices, const float* __restrict__ row_amax, int M, int E, int K,
                   int32_t* __restrict__ offsets, int32_t* __restrict__ pos, int32_t* __restrict__ row_slot,
                   int32_t* __restrict__ row_expert, float* __restrict__ seg_amax, float* __restrict__ scales_out,
                   int32_t* __restrict__ status) {
   chain_wait();
-  extern __shared__ int cnt[];            // [32 warps][E] per-warp counts -> exclusive prefixes
-  __shared__ int start[kMaxE + 1];
-  __shared__ unsigned int amax[kMaxE];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) cnt[i] = 0;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) amax[e] = 0u;
-  __syncthreads();
-  const int s = threadIdx.x;
-  int e = -1;
-  if (s < M) {
-    e = indices[s];
-    if (e < 0 || e >= E) {
-      atomicOr(status, BWMOE_STATUS_BAD_EXPERT);
-      e = -1;
-    } else if (row_amax != nullptr) {
-      atomicMax(&amax[e], __float_as_uint(row_amax[s / K]));
-    }
-  }
-  const unsigned peers = __match_any_sync(0xffffffffu, e);
-  const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
-  if (e >= 0 && rank_in_warp == 0) cnt[warp * E + e] = __popc(peers);
-  __syncthreads();
-  for (int ee = threadIdx.x; ee < E; ee += blockDim.x) {
-    int run = 0;
-    for (int w = 0; w < 32; ++w) {
-      const int c = cnt[w * E + ee];
-      cnt[w * E + ee] = run;
-      run += c;
-    }
-    start[ee + 1] = run;                 // count of expert ee, turned into an offset below
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    start[0] = 0;
-    for (int i = 0; i < E; ++i) start[i + 1] += start[i];
-  }
-  __syncthreads();
-  for (int ee = threadIdx.x; ee <= E; ee += blockDim.x) offsets[ee] = start[ee];
-  for (int ee = threadIdx.x; ee < E; ee += blockDim.x) {
-    const float a = __uint_as_float(amax[ee]);
-    if (seg_amax != nullptr) seg_amax[ee] = a;
-    if (scales_out != nullptr) scales_out[ee] = start[ee + 1] > start[ee] ? scale_from_amax(a) : 1.0f;
-  }
-  if (e >= 0) {
-    const int p = start[e] + cnt[warp * E + e] + rank_in_warp;
-    pos[s] = p;
-    row_slot[p] = s;
-    row_expert[p] = e;
-  } else if (s < M) {
-    pos[s] = -1;
-  }
-  // rows past the last segment (slots with an out-of-range expert id own none): marked as absent
-  if (s < M && s >= start[E]) row_slot[s] = -1, row_expert[s] = -1;
+  extern __shared__ int cnt[];
+  __shared__ SmallPlan sp;
+  int row;
+  const int e = small_plan(indices, row_amax, M, E, K, cnt, sp, status, true, row);
+  publish_small_plan(sp, M, E, e, row, offsets, pos, row_slot, row_expert, seg_amax, scales_out);
 }
 
 __global__ void segment_scales_kernel(const float* __restrict__ seg_amax, const int32_t* __restrict__ offsets,
@@ -228,6 +263,11 @@ __device__ __forceinline__ uint32_t e4m3x4_scaled(uint32_t w0, uint32_t w1, unsi
   return (uint32_t)lo | ((uint32_t)hi << 16);
 }
 
+__device__ __forceinline__ uint32_t e4m3x4_clamped(uint32_t w0, uint32_t w1, float s) {
+  return (uint32_t)to_e4m3x2(__uint_as_float(w0 << 16) * s, __uint_as_float(w0 & 0xffff0000u) * s) |
+         ((uint32_t)to_e4m3x2(__uint_as_float(w1 << 16) * s, __uint_as_float(w1 & 0xffff0000u) * s) << 16);
+}
+
 // Rows -> E4M3 with the scale of the row's expert.  Flat: one thread per 16 consecutive elements of
 // the [M, W] output (two 16-byte loads, one 16-byte store), the row found by one 32-bit division.
 // Measured against row-structured variants (a block or a thread group per row chunk, with and without
@@ -237,7 +277,8 @@ template <bool SRC_BY_SLOT, bool FROM_AMAX>
 __global__ void __launch_bounds__(256)
 quant_rows_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ row_slot,
                   const int32_t* __restrict__ row_expert, const float* __restrict__ scales,
-                  float* __restrict__ scales_out, unsigned M, unsigned W, int K, uint8_t* __restrict__ dst) {
+                  float* __restrict__ scales_out, unsigned M, unsigned W, int K, uint8_t* __restrict__ dst,
+                  int amax_last) {
   chain_wait();
   const unsigned per_row = W / 16;
   const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -250,7 +291,7 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restri
   const size_t srow = SRC_BY_SLOT ? (size_t)(max(row_slot[m], 0) / K) : (size_t)m;
   const uint4* in = reinterpret_cast<const uint4*>(src + srow * W) + 2 * c;
   const uint4 r0 = in[0], r1 = in[1];
-  float scale = expert >= 0 ? scales[expert] : 0.f;
+  float scale = expert >= 0 ? scales[FROM_AMAX ? min(expert, amax_last) : expert] : 0.f;
   if (FROM_AMAX && expert >= 0) {
     scale = scale_from_amax(scale);
     // published once per segment, by its first row (a store per row piled a hundred thousand stores onto a few
@@ -313,6 +354,88 @@ scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restr
     reinterpret_cast<uint4*>(dst + (size_t)row * W)[c] =
         make_uint4(e4m3x4_scaled(r0.x, r0.y, s2), e4m3x4_scaled(r0.z, r0.w, s2), e4m3x4_scaled(r1.x, r1.y, s2),
                    e4m3x4_scaled(r1.z, r1.w, s2));
+  }
+}
+
+// The plan of a decode-sized batch (at most 1024 slots) and the quantisation of its rows in one launch.  Every block
+// works the plan out for itself - the batch's routing is a few KiB and the scans take about a microsecond, less than a
+// kernel boundary - block 0 publishes it, and each block then quantises its tokens into their K rows, one thread per
+// (slot of the token, 16 elements).  A token's first pieces are requested before the plan starts.
+// GROUPS: the block-scale recipe - one scale per 128 elements, independent of the expert (eight neighbouring threads
+// share the maximum), inverse scales to x_inv; otherwise the scale of the row's segment.
+template <bool GROUPS>
+__global__ void __launch_bounds__(kPlanThreads)
+plan_quant_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ indices,
+                  const float* __restrict__ row_amax, const float* __restrict__ weights, int T, int D, int E, int K,
+                  int32_t* __restrict__ offsets, int32_t* __restrict__ pos, int32_t* __restrict__ row_slot,
+                  int32_t* __restrict__ row_expert, float* __restrict__ seg_amax, float* __restrict__ scales_out,
+                  int32_t* __restrict__ status, uint8_t* __restrict__ dst, float* __restrict__ row_w,
+                  float* __restrict__ x_inv) {
+  extern __shared__ int cnt[];
+  __shared__ SmallPlan sp;
+  __shared__ int s_row[kPlanThreads];
+  __shared__ float s_scale[kPlanThreads];          // the scale of each slot's segment
+  const int pieces = D / 16, groups = (D + 127) / 128, padded = groups * 8;     // threads of one slot: whole groups
+  const int items = K * padded;
+  // x was complete before the kernel in front of this one ran (it is an input of that kernel as well)
+  auto load_piece = [&](int t, int c, uint4& r0, uint4& r1) {
+    r0 = r1 = make_uint4(0u, 0u, 0u, 0u);
+    if (t < T && c < pieces) {
+      const uint4* in = reinterpret_cast<const uint4*>(x + (size_t)t * D) + 2 * c;
+      r0 = in[0], r1 = in[1];
+    }
+  };
+  uint4 p0, p1;
+  load_piece(blockIdx.x, (int)threadIdx.x < items ? (int)threadIdx.x % padded : pieces, p0, p1);
+  chain_wait();
+  const int M = T * K;
+  {
+    int row;
+    const int e = small_plan(indices, row_amax, M, E, K, cnt, sp, status, blockIdx.x == 0, row);
+    s_row[threadIdx.x] = row;
+    if (!GROUPS) s_scale[threadIdx.x] = e >= 0 ? scale_from_amax(__uint_as_float(sp.amax[e])) : 0.f;
+    if (blockIdx.x == 0) {
+      publish_small_plan(sp, M, E, e, row, offsets, pos, row_slot, row_expert, seg_amax, scales_out);
+      if (row_w != nullptr && e >= 0) row_w[row] = weights[threadIdx.x];   // routing weight in row order
+    }
+  }
+  __syncthreads();
+  for (int t = blockIdx.x; t < T; t += gridDim.x) {
+    for (int base = 0; base < items; base += kPlanThreads) {       // uniform for the block: the shuffles below need it
+      const int item = base + threadIdx.x;
+      const int k = item < items ? item / padded : 0, c = item < items ? item - k * padded : pieces;
+      uint4 r0 = p0, r1 = p1;
+      if (t != (int)blockIdx.x || base > 0) load_piece(t, c, r0, r1);
+      const int row = s_row[t * K + k];
+      float scale, inv = 0.f;
+      if constexpr (GROUPS) {
+        const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+        float m = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
+        for (int off = 4; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off, 8));
+        m = fmaxf(m, kGroupAmaxFloor);
+        scale = __fmul_rn(__frcp_rn(m), kFp8Max);
+        inv = __fdiv_rn(m, kFp8Max);
+      } else {
+        scale = s_scale[t * K + k];
+      }
+      if (c < pieces && row >= 0) {                  // row < 0: slot with an out-of-range expert
+        uint4 codes;
+        if constexpr (GROUPS) {                      // min/max clamp as in quant_group_rows_kernel (it decides what NaN becomes)
+          codes = make_uint4(e4m3x4_clamped(r0.x, r0.y, scale), e4m3x4_clamped(r0.z, r0.w, scale),
+                             e4m3x4_clamped(r1.x, r1.y, scale), e4m3x4_clamped(r1.z, r1.w, scale));
+          if ((c & 7) == 0) x_inv[(size_t)row * groups + (c >> 3)] = inv;
+        } else {
+          const unsigned long long s2 = splat2(scale);
+          codes = make_uint4(e4m3x4_scaled(r0.x, r0.y, s2), e4m3x4_scaled(r0.z, r0.w, s2), e4m3x4_scaled(r1.x, r1.y, s2),
+                             e4m3x4_scaled(r1.z, r1.w, s2));
+        }
+        reinterpret_cast<uint4*>(dst + (size_t)row * D)[c] = codes;
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -504,39 +627,52 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ 
   reinterpret_cast<uint4*>(out + (size_t)t * D)[v] = o;
 }
 
-// Routing of a block with S always-on experts appended as groups E .. E+S-1: every token keeps its K routed
-// slots and gets S more with weight 1.
-__global__ void append_shared_slots_kernel(const int32_t* __restrict__ idx_r, const float* __restrict__ w_r, int T,
-                                           int K, int E, int S, int32_t* __restrict__ idx, float* __restrict__ w) {
+// What the pipeline needs of a batch whose routing the caller did: max|x| of every row, the routing copied into the
+// workspace (one warp per token; `remap` turns expert ids of the whole model into slots of a resident pool, an id
+// outside [0, n_ids) or without a slot becomes -1, which the plan reports), and the words that later kernels want at
+// zero.  One launch in the place of a memset, a row-maximum kernel, a lookup kernel and one or two copies: at decode
+// sizes each of those nodes cost more than its work.
+__global__ void __launch_bounds__(256)
+routed_prepare_kernel(const __nv_bfloat16* __restrict__ x, const float* weights, const int32_t* ids,
+                      const int32_t* __restrict__ remap, int n_ids, int T, int D, int K, float* w_out, int32_t* slots,
+                      float* __restrict__ row_amax, uint32_t* __restrict__ zero, int zero_words) {
   chain_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int KS = K + S;
-  if (i >= T * KS) return;
-  const int t = i / KS, k = i - t * KS;
-  idx[i] = k < K ? idx_r[t * K + k] : E + (k - K);
-  w[i] = k < K ? w_r[t * K + k] : 1.0f;
-}
-
-// amax[first .. first+count) <- their common maximum: groups that are pieces of one tensor share its scale
-__global__ void merge_amax_kernel(float* __restrict__ amax, int first, int count) {
-  chain_wait();
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < zero_words; i += blockDim.x) zero[i] = 0u;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const size_t at = (size_t)t * K + lane;
+  if (lane < K) {                                    // K <= 32
+    const int id = ids[at];
+    slots[at] = remap == nullptr ? id : (id >= 0 && id < n_ids ? remap[id] : -1);
+    w_out[at] = weights[at];
+  }
+  if (row_amax == nullptr) return;
+  const uint4* row = reinterpret_cast<const uint4*>(x + (size_t)t * D);
   float m = 0.f;
-  for (int i = 0; i < count; ++i) m = fmaxf(m, amax[first + i]);
-  for (int i = 0; i < count; ++i) amax[first + i] = m;
+#pragma unroll 4
+  for (int v = lane; v < D / 8; v += 32) {
+    const uint4 raw = row[v];
+    const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(q[i]);
+      m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+  }
+  for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  if (lane == 0) row_amax[t] = m;
 }
 
 }  // namespace
 
-int launch_append_shared_slots(const int32_t* idx_r, const float* w_r, int T, int K, int E, int S, int32_t* idx,
-                               float* w, cudaStream_t st) {
-  const int n = T * (K + S);
-  BWMOE_CUDA_OK(launch_chained(append_shared_slots_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st, idx_r, w_r, T, K, E, S, idx, w));
-  BWMOE_CUDA_OK(cudaGetLastError());
-  return BWMOE_OK;
-}
-
-int launch_merge_amax(float* amax, int first, int count, cudaStream_t st) {
-  BWMOE_CUDA_OK(launch_chained(merge_amax_kernel, dim3(1), dim3(1), 0, st, amax, first, count));
+int launch_routed_prepare(const void* x, const float* weights, const int32_t* ids, const int32_t* remap, int n_ids, int T,
+                          int D, int K, float* w_out, int32_t* slots, float* row_amax, void* zero, size_t zero_bytes,
+                          cudaStream_t st) {
+  BWMOE_REQUIRE(T > 0 && D % 8 == 0 && K > 0 && K <= 32, BWMOE_ERR_BAD_SHAPE, "routed_prepare: T=%d D=%d K=%d", T, D, K);
+  BWMOE_CUDA_OK(launch_chained(routed_prepare_kernel, dim3(ceil_div(T, 8)), dim3(256), 0, st,
+                               static_cast<const __nv_bfloat16*>(x), weights, ids, remap, n_ids, T, D, K, w_out, slots,
+                               row_amax, static_cast<uint32_t*>(zero), (int)(zero_bytes / 4)));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }
@@ -549,6 +685,28 @@ size_t plan_scratch_bytes(int T, int E, int K) {
   return (size_t)(B * E * sizeof(int32_t) + 256);
 }
 
+inline size_t small_plan_smem(int E) { return (size_t)32 * (E + 1) * sizeof(int); }
+
+bool plan_quant_applicable(int T, int E, int K) { return (long long)T * K <= kPlanThreads && E <= kMaxE; }
+
+int launch_plan_quant(const void* x, const int32_t* indices, const float* row_amax, const float* weights, int T, int D, int E,
+                      int K, int32_t* offsets, int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax,
+                      float* scales, int32_t* status, void* xq, float* row_w, float* x_inv, cudaStream_t st) {
+  BWMOE_REQUIRE(plan_quant_applicable(T, E, K) && D % 16 == 0, BWMOE_ERR_BAD_SHAPE, "plan_quant: T=%d D=%d E=%d K=%d", T, D, E, K);
+  const dim3 grid((unsigned)std::min(T, 2 * sm_count())), block(kPlanThreads);     // two blocks of 1024 threads per SM
+  const size_t smem = small_plan_smem(E);
+  auto xb = static_cast<const __nv_bfloat16*>(x);
+  auto q = static_cast<uint8_t*>(xq);
+  if (x_inv != nullptr)
+    BWMOE_CUDA_OK(launch_chained(plan_quant_kernel<true>, grid, block, smem, st, xb, indices, row_amax, weights, T, D, E, K, offsets,
+                                 pos, row_slot, row_expert, seg_amax, scales, status, q, row_w, x_inv));
+  else
+    BWMOE_CUDA_OK(launch_chained(plan_quant_kernel<false>, grid, block, smem, st, xb, indices, row_amax, weights, T, D, E, K, offsets,
+                                 pos, row_slot, row_expert, seg_amax, scales, status, q, row_w, x_inv));
+  BWMOE_CUDA_OK(cudaGetLastError());
+  return BWMOE_OK;
+}
+
 int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                 int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,
                 void* scratch, cudaStream_t st, float* scales_out) {
@@ -559,7 +717,7 @@ int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int
                 "plan: null pointer");
   const int M = T * K;
   if (M <= kPlanThreads) {
-    BWMOE_CUDA_OK(launch_chained(plan_small_kernel, dim3(1), dim3(kPlanThreads), (size_t)32 * E * sizeof(int), st,
+    BWMOE_CUDA_OK(launch_chained(plan_small_kernel, dim3(1), dim3(kPlanThreads), small_plan_smem(E), st,
         indices, row_amax, M, E, K, offsets, pos, row_slot, row_expert, seg_amax, scales_out, status));
     BWMOE_CUDA_OK(cudaGetLastError());
     return BWMOE_OK;
@@ -632,7 +790,7 @@ int launch_gather_quant(const void* x, const int32_t* row_slot, const int32_t* r
   BWMOE_REQUIRE(x && row_slot && row_expert && scales && xq, BWMOE_ERR_NULL, "gather_quant: null pointer");
   BWMOE_REQUIRE(aligned16(x) && aligned16(xq), BWMOE_ERR_BAD_ALIGN, "gather_quant: pointers must be 16-byte aligned");
   BWMOE_CUDA_OK(launch_chained(quant_rows_kernel<true, false>, dim3(quant_grid(M, D)), dim3(256), 0, st,
-      static_cast<const __nv_bfloat16*>(x), row_slot, row_expert, scales, nullptr, M, D, K, static_cast<uint8_t*>(xq)));
+      static_cast<const __nv_bfloat16*>(x), row_slot, row_expert, scales, nullptr, M, D, K, static_cast<uint8_t*>(xq), 0));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }
@@ -650,18 +808,18 @@ int launch_scatter_quant(const void* x, const int32_t* pos, const int32_t* indic
 }
 
 int launch_requant(const void* h, const int32_t* row_expert, const float* scales_h, int M, int H,
-                   void* hq, cudaStream_t st, float* scales_from_amax_out) {
+                   void* hq, cudaStream_t st, float* scales_from_amax_out, int amax_last) {
   BWMOE_REQUIRE(M > 0 && H > 0 && H % 16 == 0, BWMOE_ERR_BAD_SHAPE, "requant: M=%d H=%d", M, H);
   BWMOE_REQUIRE(h && row_expert && scales_h && hq, BWMOE_ERR_NULL, "requant: null pointer");
   BWMOE_REQUIRE(aligned16(h) && aligned16(hq), BWMOE_ERR_BAD_ALIGN, "requant: pointers must be 16-byte aligned");
   if (scales_from_amax_out != nullptr)   // scales_h holds the segment amax; scales are derived and published
     BWMOE_CUDA_OK(launch_chained(quant_rows_kernel<false, true>, dim3(quant_grid(M, H)), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(h), nullptr,
                                                                      row_expert, scales_h, scales_from_amax_out, M, H, 1,
-                                                                     static_cast<uint8_t*>(hq)));
+                                                                     static_cast<uint8_t*>(hq), amax_last));
   else
     BWMOE_CUDA_OK(launch_chained(quant_rows_kernel<false, false>, dim3(quant_grid(M, H)), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(h), nullptr,
                                                                       row_expert, scales_h, nullptr, M, H, 1,
-                                                                      static_cast<uint8_t*>(hq)));
+                                                                      static_cast<uint8_t*>(hq), 0));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }
@@ -706,7 +864,7 @@ int launch_quant_rows_from_amax(const void* x, const int32_t* row_expert, const 
                                 void* xq, float* scales_out, cudaStream_t st) {
   BWMOE_CUDA_OK(launch_chained(quant_rows_kernel<false, true>, dim3(quant_grid(M, W)), dim3(256), 0, st,
       static_cast<const __nv_bfloat16*>(x), nullptr, row_expert, seg_amax, scales_out, M, W, 1,
-      static_cast<uint8_t*>(xq)));
+      static_cast<uint8_t*>(xq), 255));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }

@@ -40,7 +40,7 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float y) {
 // (value desc, id asc) with two warp-wide reductions: the largest key, then the lowest id that has it.
 template <int EJ>
 __device__ __forceinline__ bool select_token_regs(const float* lg_row, int E, int K, float thr_rel, float thr_abs,
-                                                  float* w_out, int32_t* i_out, int lane, float* cut_out) {
+                                                  const RouteRows& out, size_t tok, int lane) {
   unsigned key[EJ];
   float lmax = 0.f;
 #pragma unroll
@@ -76,26 +76,24 @@ __device__ __forceinline__ bool select_token_regs(const float* lg_row, int E, in
     prev = bv;
     if (it < K && lane == it) chosen_v = bv, chosen_i = bi;
   }
-  // Experts whose approximate logit lies below this cannot reach the top K whatever the rounding did
-  // (prev is the best rejected logit, or the K-th one when K == E).
-  if (cut_out != nullptr && lane == 0) *cut_out = prev - thr;
   // weights: softmax over the selected logits == softmax over all experts, renormalised
   const float top = __shfl_sync(0xffffffffu, chosen_v, 0);
   const float p = lane < K ? expf(chosen_v - top) : 0.f;
   float z = p;
   for (int off = 16; off; off >>= 1) z += __shfl_xor_sync(0xffffffffu, z, off);
   if (lane < K) {
-    w_out[lane] = p / z;
-    i_out[lane] = chosen_i;
+    out.weights[tok * out.ld + lane] = p / z;
+    out.indices[tok * out.ld + lane] = chosen_i;
   }
+  out.write_tail(tok, lane, E, K);
   return ambiguous;
 }
 __device__ __forceinline__ bool select_token(const float* lg_row, int E, int K, float thr_rel, float thr_abs,
-                                             float* w_out, int32_t* i_out, int lane, float* cut_out = nullptr) {
-  if (E <= 32) return select_token_regs<1>(lg_row, E, K, thr_rel, thr_abs, w_out, i_out, lane, cut_out);
-  if (E <= 64) return select_token_regs<2>(lg_row, E, K, thr_rel, thr_abs, w_out, i_out, lane, cut_out);
-  if (E <= 128) return select_token_regs<4>(lg_row, E, K, thr_rel, thr_abs, w_out, i_out, lane, cut_out);
-  return select_token_regs<kMaxEJ>(lg_row, E, K, thr_rel, thr_abs, w_out, i_out, lane, cut_out);
+                                             const RouteRows& out, size_t tok, int lane) {
+  if (E <= 32) return select_token_regs<1>(lg_row, E, K, thr_rel, thr_abs, out, tok, lane);
+  if (E <= 64) return select_token_regs<2>(lg_row, E, K, thr_rel, thr_abs, out, tok, lane);
+  if (E <= 128) return select_token_regs<4>(lg_row, E, K, thr_rel, thr_abs, out, tok, lane);
+  return select_token_regs<kMaxEJ>(lg_row, E, K, thr_rel, thr_abs, out, tok, lane);
 }
 
 // Exact logits of one token in fp64 by the whole block, then rounded once to fp32.
@@ -174,8 +172,9 @@ __device__ void exact_logits_block(const __nv_bfloat16* __restrict__ xrow, const
 constexpr int kTokenSmemBytes = 32 * 256 * (int)sizeof(double);     // per-warp partial logits
 __global__ void __launch_bounds__(1024)
 router_token_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int T, int D,
-                    int E, int K, float* __restrict__ weights, int32_t* __restrict__ indices,
-                    float* __restrict__ row_amax) {
+                    int E, int K, const RouteRows out, float* __restrict__ row_amax, uint32_t* __restrict__ zero,
+                    int zero_words) {
+  chain_wait();
   extern __shared__ __align__(16) double token_part[];          // [nwarps][256]
   __shared__ double lgd[256];                                   // this CTA's partial logits
   __shared__ float lg[256];
@@ -185,6 +184,9 @@ router_token_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tok = blockIdx.x / C;
   const __nv_bfloat16* xrow = x + (size_t)tok * D;
+  // words the later kernels of the call want to find at zero (a memset node of its own costs more than this)
+  if (blockIdx.x == 0)
+    for (int i = tid; i < zero_words; i += blockDim.x) zero[i] = 0u;
   int V = 1;
   while (V < E / 8) V <<= 1;
   const int NG = blockDim.x / V;                          // d-groups of this CTA
@@ -273,7 +275,7 @@ router_token_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
   if (warp == 0) {
     float m_tok = lane < nwarps ? s_max[lane] : 0.f;
     for (int off = 16; off; off >>= 1) m_tok = fmaxf(m_tok, __shfl_xor_sync(0xffffffffu, m_tok, off));
-    select_token(lg, E, K, 0.f, -1.f, weights + (size_t)tok * K, indices + (size_t)tok * K, lane);
+    select_token(lg, E, K, 0.f, -1.f, out, (size_t)tok, lane);
     if (lane == 0 && row_amax != nullptr) row_amax[tok] = m_tok;
   }
 }
@@ -286,8 +288,7 @@ router_token_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
 constexpr int kWarpTokWarps = 8;
 __global__ void __launch_bounds__(kWarpTokWarps * 32)
 router_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int T, int D,
-                   int E, int K, float* __restrict__ weights, int32_t* __restrict__ indices,
-                   float* __restrict__ row_amax) {
+                   int E, int K, const RouteRows out, float* __restrict__ row_amax) {
   __shared__ float lg[kWarpTokWarps][16];
   __shared__ float s_wnorm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -375,8 +376,7 @@ router_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   // blocks of kInner FMAs + compensated outer sum (2) + shuffle tree (<= 5)
   const float gamma = (float)(kInner + 8) * 5.9604645e-8f * 1.05f;
   const float thr_abs = 2.f * gamma * s_wnorm * sqrtf(xsq) * 1.001f;
-  const bool amb = select_token(lg[warp], E, K, 1.0e-6f, thr_abs, weights + (size_t)tok * K,
-                                indices + (size_t)tok * K, lane);
+  const bool amb = select_token(lg[warp], E, K, 1.0e-6f, thr_abs, out, (size_t)tok, lane);
   if (lane == 0 && row_amax != nullptr) row_amax[tok] = xmax;
   if (!amb) return;
   // near-tie: exact fp64 logits by this warp alone, same lane layout
@@ -404,14 +404,13 @@ router_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int j = 0; j < 8; ++j) lg[warp][8 * ev + j] = (float)a[j];
   }
   __syncwarp();
-  select_token(lg[warp], E, K, 0.f, -1.f, weights + (size_t)tok * K, indices + (size_t)tok * K, lane);
+  select_token(lg[warp], E, K, 0.f, -1.f, out, (size_t)tok, lane);
 }
 
 template <int TOK>
 __global__ void __launch_bounds__(kThreads)
 router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int T, int D,
-              int E, int K, int Epad, float* __restrict__ weights, int32_t* __restrict__ indices,
-              float* __restrict__ row_amax) {
+              int E, int K, int Epad, const RouteRows out, float* __restrict__ row_amax) {
   // xs: staged activations [kChunk][TOK] fp32; later reused for the cross-slice reduction
   // and (as doubles) for the fp64 partial sums
   __shared__ __align__(16) float xs[kThreads * TOK];
@@ -553,7 +552,7 @@ router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
     const size_t tok = tok0 + t;
     // Cauchy-Schwarz: sum_d |x_d w_de| <= |x|_2 * |w_e|_2 (s_abs holds the squared norm of x)
     const float thr_abs = 2.f * gamma * w_norm * sqrtf(s_abs[t]);
-    const bool amb = select_token(lg[t], E, K, thr_rel, thr_abs, weights + tok * K, indices + tok * K, lane);
+    const bool amb = select_token(lg[t], E, K, thr_rel, thr_abs, out, tok, lane);
     if (lane == 0) {
       if (row_amax != nullptr) row_amax[tok] = s_max[t];
       if (amb) s_flag[atomicAdd(&s_nflag, 1)] = t;
@@ -573,7 +572,7 @@ router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   for (int f = warp; f < nflag; f += kThreads / 32) {
     const int t = s_flag[f];
     const size_t tok = tok0 + t;
-    select_token(lg[t], E, K, 0.f, -1.f, weights + tok * K, indices + tok * K, lane);
+    select_token(lg[t], E, K, 0.f, -1.f, out, tok, lane);
   }
 }
 
@@ -581,8 +580,8 @@ router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 // for tokens whose candidate list overflowed.  Blocks stride over the list.
 __global__ void __launch_bounds__(256)
 router_fallback_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int D, int E,
-                       int K, float* __restrict__ weights, int32_t* __restrict__ indices,
-                       const int32_t* __restrict__ list, const int32_t* __restrict__ count) {
+                       int K, const RouteRows out, const int32_t* __restrict__ list,
+                       const int32_t* __restrict__ count) {
   chain_wait();
   __shared__ float lg[256];
   __shared__ double dsum[256];
@@ -591,19 +590,18 @@ router_fallback_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     const int tok = list[f];
     exact_logits_block(x + (size_t)tok * D, wg, D, E, lg, dsum);
     if (threadIdx.x < 32)
-      select_token(lg, E, K, 0.f, -1.f, weights + (size_t)tok * K, indices + (size_t)tok * K, threadIdx.x);
+      select_token(lg, E, K, 0.f, -1.f, out, (size_t)tok, threadIdx.x);
     __syncthreads();
   }
 }
 
 }  // namespace
 
-int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
-                           int32_t* indices, const int32_t* list, const int32_t* count, cudaStream_t st) {
+int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
+                           const int32_t* list, const int32_t* count, cudaStream_t st) {
   (void)T;
   BWMOE_CUDA_OK(launch_chained(router_fallback_kernel, dim3(64), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x),
-                                             static_cast<const __nv_bfloat16*>(wg), D, E, K, weights, indices, list,
-                                             count));
+                                             static_cast<const __nv_bfloat16*>(wg), D, E, K, out, list, count));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }
@@ -614,25 +612,30 @@ size_t router_scratch_bytes(int T, int D, int E, int K, int T_as) {
 
 int launch_router(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
                   int32_t* indices, float* row_amax, cudaStream_t st, void* scratch, size_t scratch_bytes,
-                  int32_t* status, int T_as) {
+                  int32_t* status, int T_as, int n_tail, void* zero, size_t zero_bytes) {
   const int Tc = T_as > 0 ? T_as : T;       // the batch size that picks the kernel (launch sizes follow T)
   BWMOE_REQUIRE(T > 0 && D > 0 && E > 0 && K > 0, BWMOE_ERR_BAD_SHAPE, "router: T=%d D=%d E=%d K=%d", T, D, E, K);
   BWMOE_REQUIRE(E <= 256, BWMOE_ERR_UNSUPPORTED, "router: E=%d > 256", E);
   BWMOE_REQUIRE(K <= E && K <= 32, BWMOE_ERR_UNSUPPORTED, "router: K=%d must be <= min(E,32)", K);
   BWMOE_REQUIRE(x && wg && weights && indices, BWMOE_ERR_NULL, "router: null pointer");
+  BWMOE_REQUIRE(n_tail >= 0 && K + n_tail <= 32, BWMOE_ERR_UNSUPPORTED, "router: K=%d and %d always-on slots", K, n_tail);
+  const RouteRows out{weights, indices, K + n_tail, n_tail};
   if (router_tc_applicable(Tc, D, E, K) && scratch != nullptr && scratch_bytes >= router_tc_scratch_bytes(T, D, E) &&
-      aligned16(x) && aligned16(wg))
-    return launch_router_tc(x, wg, T, D, E, K, weights, indices, row_amax, status, scratch, st);
+      aligned16(x) && aligned16(wg)) {
+    if (zero_bytes > 0) BWMOE_CUDA_OK(cudaMemsetAsync(zero, 0, zero_bytes, st));
+    return launch_router_tc(x, wg, T, D, E, K, out, row_amax, status, scratch, st);
+  }
   int Epad = 8;
   while (Epad < E) Epad <<= 1;
   auto xp = static_cast<const __nv_bfloat16*>(x);
   auto wp = static_cast<const __nv_bfloat16*>(wg);
   const bool vec_gate = (E % 8 == 0) && ((reinterpret_cast<uintptr_t>(wg) & 15u) == 0);
   const bool vec_x = (D % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+  const bool token_kernel = vec_gate && Tc < 1024 && (long long)Tc * E * D <= (1ll << 26);     // fp64 sums: small batches only
+  if (zero_bytes > 0 && !token_kernel) BWMOE_CUDA_OK(cudaMemsetAsync(zero, 0, zero_bytes, st));
   if (vec_gate && vec_x && E <= 16 && Tc >= 1024) {
-    router_warp_kernel<<<ceil_div(T, kWarpTokWarps), kWarpTokWarps * 32, 0, counted(st)>>>(xp, wp, T, D, E, K, weights,
-                                                                                 indices, row_amax);
-  } else if (vec_gate && Tc < 1024 && (long long)Tc * E * D <= (1ll << 26)) {    // fp64 sums: small batches only
+    router_warp_kernel<<<ceil_div(T, kWarpTokWarps), kWarpTokWarps * 32, 0, counted(st)>>>(xp, wp, T, D, E, K, out, row_amax);
+  } else if (token_kernel) {
     // Few tokens: a cluster of up to 8 CTAs per token (as many as keep the grid within the SMs), and enough
     // threads that every (expert octet, 8 consecutive d) pair has a thread of its own where that fits.
     static unsigned char smem_set[64] = {0};
@@ -649,21 +652,24 @@ int launch_router(const void* x, const void* wg, int T, int D, int E, int K, flo
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = kTokenSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)C;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // the kernel starts with chain_wait()
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     note_launch();
-    BWMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, router_token_kernel, xp, wp, T, D, E, K, weights, indices, row_amax));
+    BWMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, router_token_kernel, xp, wp, T, D, E, K, out, row_amax,
+                                     static_cast<uint32_t*>(zero), (int)(zero_bytes / 4)));
   } else if (Tc >= 2048) {       // both token tilings run the same arithmetic per token
     constexpr int TOK = 16;
-    router_kernel<TOK><<<ceil_div(T, TOK), kThreads, 0, counted(st)>>>(xp, wp, T, D, E, K, Epad, weights, indices, row_amax);
+    router_kernel<TOK><<<ceil_div(T, TOK), kThreads, 0, counted(st)>>>(xp, wp, T, D, E, K, Epad, out, row_amax);
   } else {
     constexpr int TOK = 4;
-    router_kernel<TOK><<<ceil_div(T, TOK), kThreads, 0, counted(st)>>>(xp, wp, T, D, E, K, Epad, weights, indices, row_amax);
+    router_kernel<TOK><<<ceil_div(T, TOK), kThreads, 0, counted(st)>>>(xp, wp, T, D, E, K, Epad, out, row_amax);
   }
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;

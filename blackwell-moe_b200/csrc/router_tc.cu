@@ -231,9 +231,8 @@ template <int EJ>   // 32 * EJ >= E: logits each lane holds
 __global__ void __launch_bounds__(256)
 refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wgt,
               const float* __restrict__ wnorm2, const float* __restrict__ logits, int ld_logits, int T, int D,
-              int E, int K, float* __restrict__ weights, int32_t* __restrict__ indices,
-              float* __restrict__ row_amax, int32_t* __restrict__ fallback_count,
-              int32_t* __restrict__ fallback_list) {
+              int E, int K, const RouteRows out, float* __restrict__ row_amax,
+              int32_t* __restrict__ fallback_count, int32_t* __restrict__ fallback_list) {
   chain_wait();
   const int lane = threadIdx.x & 31;
   const int tok = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -384,9 +383,10 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   float z = pexp;
   for (int off = 16; off; off >>= 1) z += __shfl_xor_sync(0xffffffffu, z, off);
   if (chosen) {
-    weights[(size_t)tok * K + rank] = pexp / z;
-    indices[(size_t)tok * K + rank] = ci;
+    out.weights[(size_t)tok * out.ld + rank] = pexp / z;
+    out.indices[(size_t)tok * out.ld + rank] = ci;
   }
+  out.write_tail((size_t)tok, lane, E, K);
 }
 
 int make_map_bf16(CUtensorMap* map, const void* base, int rows, int cols, int box_cols, int box_rows) {
@@ -434,10 +434,10 @@ bool router_tc_applicable(int T, int D, int E, int K) {
 size_t router_tc_scratch_bytes(int T, int D, int E) { return tc_layout(T, D, E).total; }
 
 // Exact router for the tokens the candidate list could not settle (device list, count read on the device).
-int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
-                           int32_t* indices, const int32_t* list, const int32_t* count, cudaStream_t st);
+int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
+                           const int32_t* list, const int32_t* count, cudaStream_t st);
 
-int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, float* weights, int32_t* indices,
+int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
                      float* row_amax, int32_t* status, void* scratch, cudaStream_t st) {
   BWMOE_REQUIRE(scratch != nullptr && aligned16(scratch), BWMOE_ERR_WORKSPACE, "router: scratch buffer required");
   BWMOE_REQUIRE(aligned16(x) && aligned16(wg), BWMOE_ERR_BAD_ALIGN, "router: pointers must be 16-byte aligned");
@@ -468,19 +468,19 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
   auto xb = static_cast<const __nv_bfloat16*>(x);
   const unsigned rgrid = (unsigned)ceil_div(T, 8);
   if (E <= 32)
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<1>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, weights, indices, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<1>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   else if (E <= 64)
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<2>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, weights, indices, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<2>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   else if (E <= 128)
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<4>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, weights, indices, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<4>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   else
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<8>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, weights, indices, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<8>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   BWMOE_CUDA_OK(cudaGetLastError());
-  return launch_router_fallback(x, wg, T, D, E, K, weights, indices, fb_list, fb_count, st);
+  return launch_router_fallback(x, wg, T, D, E, K, out, fb_list, fb_count, st);
 }
 
 }  // namespace bwmoe
