@@ -223,7 +223,7 @@ int run_pipeline(const void* x, const float* weights, const int32_t* indices, co
       return rc;
   } else {
     if ((rc = launch_plan(indices, row_amax, T, E, K, offsets, pos, row_slot, row_expert, amax_x, status,
-                          at<void>(ws, L.plan_scratch), st, scale_x)))
+                          at<void>(ws, L.plan_scratch), st, scale_x, /*amax_is_zero=*/true)))
       return rc;
     if ((rc = launch_scatter_quant(x, pos, indices, scale_x, T, D, K, at<void>(ws, L.xq), st, weights, row_w))) return rc;
   }

@@ -145,7 +145,7 @@ int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, i
 size_t plan_scratch_bytes(int T, int E, int K);
 int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                 int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,
-                void* scratch, cudaStream_t st, float* scales_out = nullptr);
+                void* scratch, cudaStream_t st, float* scales_out = nullptr, bool amax_is_zero = false);
 // Plan and quantisation of a decode-sized batch in one launch (x_inv != nullptr: the block-scale recipe).  Only inside
 // the whole-block forwards: x is read before the kernel in front of it has finished.
 bool plan_quant_applicable(int T, int E, int K);

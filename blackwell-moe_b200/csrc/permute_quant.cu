@@ -14,20 +14,27 @@ namespace bwmoe {
 namespace {
 
 constexpr int kPlanThreads = 1024;
-constexpr int kSlotsPerBlock = 4096;   // slots ranked by one block (4 rounds of 1024)
 constexpr int kMaxE = 256;
+constexpr int kPlanMaxBlocks = 256;
+// Slots ranked by one block, in rounds of 1024: two rounds while that keeps the blocks at 256 or fewer (a prefill batch
+// then covers the chip), more beyond, because every block adds up all blocks' histograms.
+inline int plan_slots_per_block(long long M) {
+  const long long per = (M + kPlanMaxBlocks - 1) / kPlanMaxBlocks;
+  return (int)(per <= 2 * kPlanThreads ? 2 * kPlanThreads : (per + kPlanThreads - 1) / kPlanThreads * kPlanThreads);
+}
 
 // ---- pass 1: per-block histogram of expert ids + per-segment max of the row amax ----
 __global__ void __launch_bounds__(kPlanThreads)
 plan_hist_kernel(const int32_t* __restrict__ indices, const float* __restrict__ row_amax, int M, int E,
-                 int K, int32_t* __restrict__ block_hist, float* __restrict__ seg_amax,
+                 int K, int per_block, int32_t* __restrict__ block_hist, float* __restrict__ seg_amax,
                  int32_t* __restrict__ status) {
+  chain_wait();
   __shared__ int hist[kMaxE];
   __shared__ unsigned int amax[kMaxE];
   for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0, amax[e] = 0u;
   __syncthreads();
-  const int s0 = blockIdx.x * kSlotsPerBlock;
-  for (int i = threadIdx.x; i < kSlotsPerBlock; i += blockDim.x) {
+  const int s0 = blockIdx.x * per_block;
+  for (int i = threadIdx.x; i < per_block; i += blockDim.x) {
     const int s = s0 + i;
     if (s >= M) break;
     const int e = indices[s];
@@ -45,77 +52,96 @@ plan_hist_kernel(const int32_t* __restrict__ indices, const float* __restrict__ 
   }
 }
 
-// ---- pass 2: offsets[E+1] and, per block, the first row of each expert's slots ----
-__global__ void __launch_bounds__(kMaxE)
-plan_scan_kernel(int32_t* __restrict__ block_hist, int B, int E, int32_t* __restrict__ offsets) {
-  __shared__ int total[kMaxE];
-  __shared__ int start[kMaxE + 1];
-  const int e = threadIdx.x;
-  if (e < E) {
-    int run = 0;
-    for (int b = 0; b < B; ++b) {
-      const int c = block_hist[(size_t)b * E + e];
-      block_hist[(size_t)b * E + e] = run;   // exclusive prefix over blocks
-      run += c;
-    }
-    total[e] = run;
-  }
-  __syncthreads();
-  if (e == 0) {
-    int run = 0;
-    for (int i = 0; i < E; ++i) {
-      start[i] = run;
-      run += total[i];
-    }
-    start[E] = run;
-  }
-  __syncthreads();
-  if (e < E) offsets[e] = start[e];
-  if (e == 0) offsets[E] = start[E];
-  if (e < E) {
-    const int base = start[e];
-    for (int b = 0; b < B; ++b) block_hist[(size_t)b * E + e] += base;
-  }
-}
-
-// ---- pass 3: stable rank of every slot inside its block -> permuted row ----
+// ---- pass 2: segment offsets, then the stable rank of every slot -> permuted row ----
+// Every block adds up the histograms for itself - all of them for the offsets, those of the blocks before it for the
+// place of its own first slot of each expert (four threads per expert, independent loads; at 128 blocks x 256 experts
+// 128 KiB from L2) - so no one-block scan kernel sits between the passes, and block 0 publishes offsets and scales.
+// The counts of the 32 warps are scanned with shuffles, one expert per warp at a time (a thread that walks 32 dependent
+// shared-memory sums takes ~1000 cycles per round).
 __global__ void __launch_bounds__(kPlanThreads)
-plan_rank_kernel(const int32_t* __restrict__ indices, int M, int E, const int32_t* __restrict__ block_base,
-                 const int32_t* __restrict__ offsets, int32_t* __restrict__ pos, int32_t* __restrict__ row_slot,
-                 int32_t* __restrict__ row_expert) {
-  extern __shared__ int cnt[];            // [32 warps][E] counts of this pass, then exclusive prefixes
-  __shared__ int round_base[kMaxE];       // slots of earlier rounds in this block, per expert
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n_rows = offsets[E];          // rows that exist (slots with a valid expert id)
-  for (int e = threadIdx.x; e < E; e += blockDim.x) round_base[e] = block_base[(size_t)blockIdx.x * E + e];
-  const int s0 = blockIdx.x * kSlotsPerBlock;
-  for (int r = 0; r < kSlotsPerBlock / kPlanThreads; ++r) {
+plan_rank_kernel(const int32_t* __restrict__ indices, int M, int E, int per_block, int B,
+                 const int32_t* __restrict__ block_hist, const float* __restrict__ seg_amax,
+                 int32_t* __restrict__ offsets, float* __restrict__ scales_out, int32_t* __restrict__ pos,
+                 int32_t* __restrict__ row_slot, int32_t* __restrict__ row_expert) {
+  chain_wait();
+  extern __shared__ int cnt[];            // [32 warps][E + 1] counts of a round, then exclusive prefixes
+  __shared__ int part[2][4][kMaxE];       // [all blocks | blocks before this one][quarter][expert]
+  __shared__ int start[kMaxE + 1];
+  __shared__ int round_base[kMaxE];       // next row of each expert for this block's slots
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ld = E + 1;
+  {
+    const int ee = threadIdx.x % kMaxE, q = threadIdx.x / kMaxE;
+    int all = 0, before = 0;
+    if (ee < E) {
+#pragma unroll 8
+      for (int b = q; b < B; b += 4) {
+        const int c = block_hist[(size_t)b * E + ee];
+        all += c;
+        if (b < (int)blockIdx.x) before += c;
+      }
+    }
+    part[0][q][ee] = all, part[1][q][ee] = before;
+  }
+  __syncthreads();
+  if (warp == 0) {                        // offsets: eight experts per lane, then a scan of the lane totals
+    int v[kMaxE / 32], run = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxE / 32; ++j) {
+      const int ee = lane * (kMaxE / 32) + j;
+      run += part[0][0][ee] + part[0][1][ee] + part[0][2][ee] + part[0][3][ee];
+      v[j] = run;
+    }
+    int incl = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+#pragma unroll
+    for (int j = 0; j < kMaxE / 32; ++j) start[lane * (kMaxE / 32) + j + 1] = incl - run + v[j];
+    if (lane == 0) start[0] = 0;
+  }
+  __syncthreads();
+  const int n_rows = start[E];            // rows that exist (slots with a valid expert id)
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    round_base[e] = start[e] + part[1][0][e] + part[1][1][e] + part[1][2][e] + part[1][3][e];
+    if (blockIdx.x == 0) {
+      offsets[e] = start[e];
+      if (e == 0) offsets[E] = n_rows;
+      if (scales_out != nullptr) scales_out[e] = start[e + 1] > start[e] ? scale_from_amax(seg_amax[e]) : 1.0f;
+    }
+  }
+  const int s0 = blockIdx.x * per_block;
+  for (int r = 0; r < per_block / kPlanThreads; ++r) {
     if (s0 + r * kPlanThreads >= M) break;   // uniform for the block
-    for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) cnt[i] = 0;
-    __syncthreads();
     const int s = s0 + r * kPlanThreads + threadIdx.x;
     int e = -1;
     if (s < M) {
       e = indices[s];
       if (e < 0 || e >= E) e = -1;
     }
+    for (int i = threadIdx.x; i < 32 * ld; i += blockDim.x) cnt[i] = 0;
     const unsigned peers = __match_any_sync(0xffffffffu, e);
     const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
-    if (e >= 0 && rank_in_warp == 0) cnt[warp * E + e] = __popc(peers);
     __syncthreads();
-    for (int ee = threadIdx.x; ee < E; ee += blockDim.x) {
-      int run = 0;
-      for (int w = 0; w < 32; ++w) {
-        const int c = cnt[w * E + ee];
-        cnt[w * E + ee] = run;
-        run += c;
+    if (e >= 0 && rank_in_warp == 0) cnt[warp * ld + e] = __popc(peers);
+    __syncthreads();
+    for (int ee = warp; ee < E; ee += 32) {
+      const int c = cnt[lane * ld + ee];
+      int incl = c;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
       }
-      // total of this pass is added to round_base after everyone has read it
-      cnt[32 * E + ee] = run;
+      const int base = round_base[ee];
+      cnt[lane * ld + ee] = base + incl - c;
+      __syncwarp();
+      if (lane == 31) round_base[ee] = base + incl;      // the next round's
     }
     __syncthreads();
     if (e >= 0) {
-      const int p = round_base[e] + cnt[warp * E + e] + rank_in_warp;
+      const int p = cnt[warp * ld + e] + rank_in_warp;
       pos[s] = p;
       row_slot[p] = s;
       row_expert[p] = e;
@@ -125,8 +151,6 @@ plan_rank_kernel(const int32_t* __restrict__ indices, int M, int E, const int32_
     // slots with an expert id out of range own no row: the rows past the last segment are marked
     // so that the row-wise kernels behind the plan skip them
     if (s < M && s >= n_rows) row_slot[s] = -1, row_expert[s] = -1;
-    __syncthreads();
-    for (int ee = threadIdx.x; ee < E; ee += blockDim.x) round_base[ee] += cnt[32 * E + ee];
     __syncthreads();
   }
 }
@@ -681,7 +705,7 @@ inline unsigned quant_grid(int M, int W) { return (unsigned)(((size_t)M * (W / 1
 
 size_t plan_scratch_bytes(int T, int E, int K) {
   const long long M = (long long)T * K;
-  const long long B = (M + kSlotsPerBlock - 1) / kSlotsPerBlock;
+  const long long per = plan_slots_per_block(M), B = (M + per - 1) / per;
   return (size_t)(B * E * sizeof(int32_t) + 256);
 }
 
@@ -709,7 +733,7 @@ int launch_plan_quant(const void* x, const int32_t* indices, const float* row_am
 
 int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                 int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,
-                void* scratch, cudaStream_t st, float* scales_out) {
+                void* scratch, cudaStream_t st, float* scales_out, bool amax_is_zero) {
   BWMOE_REQUIRE(T > 0 && E > 0 && K > 0, BWMOE_ERR_BAD_SHAPE, "plan: T=%d E=%d K=%d", T, E, K);
   BWMOE_REQUIRE(E <= kMaxE, BWMOE_ERR_UNSUPPORTED, "plan: E=%d > %d", E, kMaxE);
   BWMOE_REQUIRE((long long)T * K < (1ll << 31), BWMOE_ERR_UNSUPPORTED, "plan: T*K too large");
@@ -722,31 +746,30 @@ int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int
     BWMOE_CUDA_OK(cudaGetLastError());
     return BWMOE_OK;
   }
-  const int B = ceil_div(M, kSlotsPerBlock);
+  const int per_block = plan_slots_per_block(M), B = ceil_div(M, per_block);
   int32_t* block_hist = static_cast<int32_t*>(scratch);
-  if (seg_amax != nullptr) BWMOE_CUDA_OK(cudaMemsetAsync(seg_amax, 0, sizeof(float) * E, st));
-  plan_hist_kernel<<<B, kPlanThreads, 0, counted(st)>>>(indices, row_amax, M, E, K, block_hist,
-                                               row_amax ? seg_amax : nullptr, status);
-  plan_scan_kernel<<<1, kMaxE, 0, counted(st)>>>(block_hist, B, E, offsets);
-  const size_t smem = (size_t)33 * E * sizeof(int);
-  plan_rank_kernel<<<B, kPlanThreads, smem, counted(st)>>>(indices, M, E, block_hist, offsets, pos, row_slot, row_expert);
+  if (seg_amax != nullptr && !amax_is_zero) BWMOE_CUDA_OK(cudaMemsetAsync(seg_amax, 0, sizeof(float) * E, st));
+  BWMOE_CUDA_OK(launch_chained(plan_hist_kernel, dim3(B), dim3(kPlanThreads), 0, st, indices, row_amax, M, E, K, per_block,
+                               block_hist, row_amax ? seg_amax : nullptr, status));
+  BWMOE_CUDA_OK(launch_chained(plan_rank_kernel, dim3(B), dim3(kPlanThreads), small_plan_smem(E), st, indices, M, E, per_block, B,
+                               block_hist, seg_amax, offsets, scales_out, pos, row_slot, row_expert));
   BWMOE_CUDA_OK(cudaGetLastError());
-  if (scales_out != nullptr) return launch_segment_scales(seg_amax, offsets, E, scales_out, st);
   return BWMOE_OK;
 }
 
 // ---- allocation-free variant of the permutation plan ------------------------------
 // Scratch for callers that cannot hand the library a scratch buffer: a fixed array
 // that lives in every GPU's memory from the moment the library is loaded there.
-constexpr int kStaticPlanBlocks = 64;                       // 64 * 4096 = 262144 slots at most
-static __device__ __align__(256) int32_t g_static_plan_scratch[kStaticPlanBlocks * kMaxE];   // 64 KiB
+constexpr int kStaticPlanSlots = 262144;                     // slots at most: 128 blocks of 2048
+constexpr int kStaticPlanBlocks = kStaticPlanSlots / (2 * kPlanThreads);
+static __device__ __align__(256) int32_t g_static_plan_scratch[kStaticPlanBlocks * kMaxE];   // 128 KiB
 
 int launch_plan_static(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                        int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,
                        cudaStream_t st) {
   BWMOE_REQUIRE(T > 0 && E > 0 && K > 0, BWMOE_ERR_BAD_SHAPE, "plan_static: T=%d E=%d K=%d", T, E, K);
   BWMOE_REQUIRE(E <= kMaxE, BWMOE_ERR_UNSUPPORTED, "plan_static: E=%d > %d", E, kMaxE);
-  const long long max_slots = (long long)kStaticPlanBlocks * kSlotsPerBlock;
+  const long long max_slots = kStaticPlanSlots;
   BWMOE_REQUIRE((long long)T * K <= max_slots, BWMOE_ERR_UNSUPPORTED,
                 "plan_static: T*K=%lld exceeds the %lld slots the built-in scratch covers; "
                 "use bwmoe_permute_plan with a caller-provided scratch buffer",

@@ -338,7 +338,7 @@ int bwmoe_permute_plan(const int32_t* d_indices, const float* d_row_amax, int T,
  * framework's allocator callback or out-of-memory handler, a plugin that was handed
  * only its input and output buffers, a real-time loop that has frozen its memory
  * pool.  (No counterpart in the reference, which allocates freely through torch.)
- * The scratch is a 64 KiB array built into the library image; every GPU that loads
+ * The scratch is a 128 KiB array built into the library image; every GPU that loads
  * the library holds it until the process exits.  Limits and rules:
  *   - T*K <= 262144 slots and E <= 256; larger requests fail with
  *     BWMOE_ERR_UNSUPPORTED and a message pointing to bwmoe_permute_plan.
