@@ -37,9 +37,19 @@ inline cudaStream_t counted(cudaStream_t st) {
 // kernel it depends on has completed and its writes are visible.  A kernel that calls chain_wait() may
 // also be launched the ordinary way (the instruction then returns at once), but a kernel launched through
 // launch_chained() MUST call it.
+//
+// chain_next(), called AFTER chain_wait(), lets the next kernel of the chain be scheduled as soon as every block of
+// this one has got that far: its blocks take the places that are free (or become free) and do what needs no
+// result of this kernel while this kernel still runs.  Since every kernel signals only behind its own wait, a
+// kernel that has been scheduled knows that everything BEFORE its direct predecessor is complete and visible.
 __device__ __forceinline__ void chain_wait() {
 #if defined(__CUDA_ARCH__)
   asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void chain_next() {
+#if defined(__CUDA_ARCH__)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #endif
 }
 template <typename... KArgs, typename... Args>

@@ -1,7 +1,8 @@
 // Router for wide gates and large batches: logits on the tensor cores, selection exact.
 //
 // Same contract as the other router kernels (selection on the exactly-rounded fp32 logits,
-// ties to the lower expert id; role of src/blackwell_moe/kernels/routing.py:14-79).  Three steps:
+// ties to the lower expert id; role of src/blackwell_moe/kernels/routing.py:14-79).  Three steps, of which the
+// transposition is launched second and runs beside the tensor-core logits (neither needs the other):
 //   1. transpose_gate_kernel : w_gate[D,E] -> w_gate^T[E,D] (so that one expert's column is
 //                              contiguous) and the squared column norms
 //   2. tc_logits_kernel      : logits = x . w_gate with tcgen05.mma kind::f16 (bf16 inputs, fp32
@@ -9,14 +10,14 @@
 //   3. refine_kernel         : one warp per token.  Warp-wide selection of the 12 best tensor-core
 //                              logits, sorted.  Those logits are only trusted to
 //                              t = 2^-14 * |x|_2 * |w_e|_2 (four times the worst case of a
-//                              truncating fp32 accumulation of 4096 products).  Every expert within
-//                              2t of the K-th best is a candidate; candidates more than 2t apart are
-//                              certainly in the right order already.  Runs of candidates that are
-//                              closer than 2t to a neighbour are recomputed with the blocked
+//                              truncating fp32 accumulation of 4096 products).  Every expert that may
+//                              still reach the K-th best is a candidate; candidates further apart than the
+//                              sum of their t are certainly in the right order already.  Candidates that are
+//                              closer than that to another one are recomputed with the blocked
 //                              compensated fp32 sum of the SIMT routers (error bound known), and in
 //                              fp64 if still within that bound of each other; the final top-K is
-//                              read off the mixed list.  A token whose 12 best all fall within the
-//                              cut is recomputed over all experts by the exact fallback kernel.
+//                              read off the mixed list.  A token for which an expert beyond the 12 best
+//                              may be a candidate is recomputed over all experts by the exact fallback kernel.
 // An expert outside the candidate set has an exact logit below that of K candidates, so the
 // result equals the exact selection.
 #include "sm100_gemm.cuh"
@@ -38,7 +39,8 @@ constexpr float kTcTrust = 6.103515625e-05f;   // 2^-14
 __global__ void __launch_bounds__(256)
 transpose_gate_kernel(const __nv_bfloat16* __restrict__ wg, int D, int E, __nv_bfloat16* __restrict__ wgt,
                       float* __restrict__ wnorm2) {
-  chain_wait();
+  // Launched behind tc_logits_kernel, of which it needs nothing: once scheduled, everything before that kernel is
+  // complete (the cleared norms, the last readers of wgt), so the work comes first and the wait last.
   __shared__ __nv_bfloat16 tile[32][33];
   const int d0 = blockIdx.x * 32, e0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;     // 32 x 8
@@ -56,6 +58,7 @@ transpose_gate_kernel(const __nv_bfloat16* __restrict__ wg, int D, int E, __nv_b
     for (int off = 16; off; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
     if (tx == 0 && e < E) atomicAdd(wnorm2 + e, sq);          // feeds thresholds only: order irrelevant
   }
+  chain_wait();                // this kernel's end must not come before the logits are there
 }
 
 // ---- 2. tensor-core logits + per-token candidate list ------------------------------------
@@ -86,6 +89,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 tc_logits_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const TcParams p) {
   chain_wait();
+  chain_next();             // transpose_gate_kernel runs beside this one
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
@@ -240,7 +244,8 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   const __nv_bfloat16* xrow = x + (size_t)tok * D;
 
   // ---- |x|_2, max|x|, largest column norm ----
-  float xsq = 0.f, xmax = 0.f;
+  float xsq = 0.f;
+  __nv_bfloat162 xmax2 = __floats2bfloat162_rn(0.f, 0.f);
   for (int d0 = lane * 8; d0 < D; d0 += 256) {
     const uint4 raw = *reinterpret_cast<const uint4*>(xrow + d0);
     const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -248,18 +253,21 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
     for (int j = 0; j < 4; ++j) {
       const float2 f = __bfloat1622float2(px[j]);
       xsq = fmaf(f.x, f.x, fmaf(f.y, f.y, xsq));
-      xmax = fmaxf(xmax, fmaxf(fabsf(f.x), fabsf(f.y)));
     }
+    if (row_amax != nullptr)           // (per-tensor recipe; |x| of a pair at a time: both are exact in bf16)
+      xmax2 = __hmax2(xmax2, __hmax2(__hmax2(__habs2(px[0]), __habs2(px[1])), __hmax2(__habs2(px[2]), __habs2(px[3]))));
   }
-  for (int off = 16; off; off >>= 1) {
-    xsq += __shfl_xor_sync(0xffffffffu, xsq, off);
-    xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, off));
+  for (int off = 16; off; off >>= 1) xsq += __shfl_xor_sync(0xffffffffu, xsq, off);
+  if (row_amax != nullptr) {
+    float xmax = fmaxf(__low2float(xmax2), __high2float(xmax2));
+    for (int off = 16; off; off >>= 1) xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, off));
+    if (lane == 0) row_amax[tok] = xmax;
   }
-  if (lane == 0 && row_amax != nullptr) row_amax[tok] = xmax;
-  float wn2 = 0.f;
+  float wn2 = 0.f;                                        // the largest squared column norm
   for (int e = lane; e < E; e += 32) wn2 = fmaxf(wn2, wnorm2[e]);
   for (int off = 16; off; off >>= 1) wn2 = fmaxf(wn2, __shfl_xor_sync(0xffffffffu, wn2, off));
-  const float xw = sqrtf(xsq) * sqrtf(wn2) * 1.002f;      // >= sum_d |x_d w_de| for every expert
+  const float xnorm = sqrtf(xsq) * 1.002f;
+  const float xw = xnorm * sqrtf(wn2);                    // >= sum_d |x_d w_de| for every expert
   const float t2 = 2.f * kTcTrust * xw;                   // two logits further apart are ordered for sure
 
   // ---- the best tensor-core logits, sorted by (value desc, id asc): lane j keeps entry j.  The list
@@ -298,20 +306,40 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
     if (it >= K && bv < kth_tc - t2) break;      // warp-uniform: bv is the same in every lane
   }
 
-  // ---- candidates: the list prefix within 2t of the K-th entry ----
+  // ---- candidates.  An entry is trusted to t = 2^-14 |x| |w_e| of its OWN expert: with one bound for all, a single
+  //      popular expert (whose column is several times as long) makes every other pair look close, and tokens end up
+  //      on the all-expert path (8192 tokens of a skewed 128-expert router: 35 us there).  `low` is a lower bound of the
+  //      exact K-th best; what cannot reach it is out. ----
   const float kth = __shfl_sync(0xffffffffu, cv, K - 1);
-  const unsigned in_mask = __ballot_sync(0xffffffffu, lane < n_list && cv >= kth - t2);
-  const int n_cand = __popc(in_mask);
-  if (n_cand >= L_CAND && E > L_CAND) {
-    // the list may be missing experts that are just as close: all-expert exact kernel
-    if (lane == 0) fallback_list[atomicAdd(fallback_count, 1)] = tok;
+  const float t_mine = lane < n_list ? kTcTrust * xnorm * sqrtf(wnorm2[ci]) : 0.f;
+  float low = lane < K ? cv - t_mine : INFINITY;
+  for (int off = 16; off; off >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, off));
+  const unsigned in_mask = __ballot_sync(0xffffffffu, lane < n_list && cv + t_mine >= low);
+  bool settled = (in_mask & ((1u << K) - 1u)) == (1u << K) - 1u;      // (not so with NaN or infinite logits)
+  if (n_list == L_CAND && E > L_CAND && settled) {        // the list was cut off: could an expert outside it be a candidate?
+    float rest = 0.f;                                     // the longest column among those
+#pragma unroll
+    for (int j = 0; j < EJ; ++j)
+      if (key[j] != 0u) rest = fmaxf(rest, wnorm2[lane + 32 * j]);
+    for (int off = 16; off; off >>= 1) rest = fmaxf(rest, __shfl_xor_sync(0xffffffffu, rest, off));
+    settled = __shfl_sync(0xffffffffu, cv, L_CAND - 1) + kTcTrust * xnorm * sqrtf(rest) < low;
+  }
+  if (!settled) {
+    if (lane == 0) fallback_list[atomicAdd(fallback_count, 1)] = tok;      // all-expert exact kernel
     return;
   }
-  // ---- runs of candidates closer than 2t to a neighbour need exact logits ----
-  const float prev = __shfl_up_sync(0xffffffffu, cv, 1);
-  const bool close_up = lane > 0 && lane < n_cand && prev - cv <= t2;
-  const unsigned up_mask = __ballot_sync(0xffffffffu, close_up);
-  const unsigned redo = (up_mask | (up_mask >> 1)) & ((1u << n_cand) - 1u);   // both members of every close pair
+  // ---- candidates whose error intervals overlap need exact logits.  Neighbours in the list tell whether there are any
+  //      such pairs at all; only then all pairs are looked at. ----
+  unsigned redo = 0u;
+  const float above = __shfl_up_sync(0xffffffffu, cv, 1);
+  if (__any_sync(0xffffffffu, lane > 0 && ((in_mask >> lane) & 1u) && above - cv <= t_mine + kTcTrust * xw)) {
+    bool close = false;
+    for (int c = 0; c < n_list; ++c) {
+      const float vc = __shfl_sync(0xffffffffu, cv, c), tc = __shfl_sync(0xffffffffu, t_mine, c);
+      close |= c != lane && ((in_mask >> c) & 1u) && fabsf(vc - cv) <= tc + t_mine;
+    }
+    redo = __ballot_sync(0xffffffffu, close) & in_mask;
+  }
   float mine = cv;
   if (redo != 0u) {
     // one candidate at a time (usually two or three): x is re-read from L1, few registers are live
@@ -359,7 +387,7 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       exact |= __ballot_sync(0xffffffffu, hit);
     }
 #pragma unroll 1
-    for (int c = 0; c < n_cand; ++c) {
+    for (int c = 0; c < n_list; ++c) {
       if (!((exact >> c) & 1u)) continue;
       const int e = __shfl_sync(0xffffffffu, ci, c);
       double a = 0.0;
@@ -374,9 +402,9 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   for (int c = 0; c < L_CAND; ++c) {
     const float vc = __shfl_sync(0xffffffffu, mine, c);
     const int ic = __shfl_sync(0xffffffffu, ci, c);
-    if (c < n_cand && (vc > mine || (vc == mine && ic < ci))) ++rank;
+    if (((in_mask >> c) & 1u) && (vc > mine || (vc == mine && ic < ci))) ++rank;
   }
-  const bool chosen = lane < n_cand && rank < K;
+  const bool chosen = ((in_mask >> lane) & 1u) && rank < K;
   float top = chosen && rank == 0 ? mine : -INFINITY;
   for (int off = 16; off; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
   const float pexp = chosen ? expf(mine - top) : 0.f;
@@ -450,10 +478,6 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
   auto* fb_list = reinterpret_cast<int32_t*>(base + L.fb_list);
   BWMOE_CUDA_OK(cudaMemsetAsync(base, 0, L.wgt, st));        // column norms, fallback counter, private status word
   if (status == nullptr) status = fb_count + 1;
-  BWMOE_CUDA_OK(launch_chained(transpose_gate_kernel, dim3(ceil_div(D, 32), ceil_div(E, 32)), dim3(256), 0, st,
-                               static_cast<const __nv_bfloat16*>(wg), D, E, wgt, wnorm2));
-  BWMOE_CUDA_OK(cudaGetLastError());
-
   CUtensorMap mx, mw;
   if (int rc = make_map_bf16(&mx, x, T, D, R_BK, BM)) return rc;
   if (int rc = make_map_bf16(&mw, wg, D, E, 64, R_BK)) return rc;
@@ -464,6 +488,9 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
   p.split_n = (p.n_chunks > 1 && ceil_div(T, BM) * p.n_chunks * 2 <= sm_count()) ? 1 : 0;
   const int grid = std::min(sm_count(), ceil_div(T, BM) * (p.split_n ? p.n_chunks : 1));
   BWMOE_CUDA_OK(launch_chained(tc_logits_kernel, dim3(grid), dim3(NUM_THREADS), R_SMEM_BYTES, st, mx, mw, p));
+  BWMOE_CUDA_OK(cudaGetLastError());
+  BWMOE_CUDA_OK(launch_chained(transpose_gate_kernel, dim3(ceil_div(D, 32), ceil_div(E, 32)), dim3(256), 0, st,
+                               static_cast<const __nv_bfloat16*>(wg), D, E, wgt, wnorm2));
   BWMOE_CUDA_OK(cudaGetLastError());
   auto xb = static_cast<const __nv_bfloat16*>(x);
   const unsigned rgrid = (unsigned)ceil_div(T, 8);
