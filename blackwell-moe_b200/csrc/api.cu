@@ -227,7 +227,7 @@ int run_pipeline(const void* x, const float* weights, const int32_t* indices, co
       return rc;
     if ((rc = launch_scatter_quant(x, pos, indices, scale_x, T, D, K, at<void>(ws, L.xq), st, weights, row_w))) return rc;
   }
-  const FusedRequant fr{at<void>(ws, L.hq), scale_h, at<unsigned int>(ws, L.arrivals)};
+  const FusedRequant fr{at<void>(ws, L.hq), scale_h, at<unsigned int>(ws, L.arrivals), row_expert};
   bool requant_done = false;
   if ((rc = launch_gateup(at<void>(ws, L.xq), offsets, scale_x, wg, wu, sg, su, M, D, H, E, at<void>(ws, L.h),
                           amax_h, status, at<void>(ws, L.gemm_scratch), st, &fr, &requant_done, n_shared)))
@@ -240,6 +240,7 @@ int run_pipeline(const void* x, const float* weights, const int32_t* indices, co
   CombineArgs ca{pos, weights, T, K, out, out_scale, residual};
   ca.row_w = row_w;
   ca.row_slot = row_slot;
+  ca.row_expert = row_expert;
   ca.n_tail = n_shared;
   ca.reduce = (flags & BWMOE_FLAG_REDUCE_COMBINE) != 0 && out_scale == 1.0f && residual == nullptr && M > 64;
   if (ca.reduce) BWMOE_CUDA_OK(cudaMemsetAsync(out, 0, (size_t)T * D * 2, st));   // the epilogue adds into it
@@ -515,7 +516,8 @@ int bwmoe_dense_mlp(const void* x, const void* wg, const void* wu, const void* w
   if ((rc = launch_quant_rows_from_amax(x, at<int32_t>(ws, L.row_expert), at<float>(ws, L.amax_x), T, D,
                                         at<void>(ws, L.xq), at<float>(ws, L.scale_x), st)))
     return rc;
-  const FusedRequant fr{at<void>(ws, L.hq), at<float>(ws, L.scale_h), at<unsigned int>(ws, L.arrivals)};
+  const FusedRequant fr{at<void>(ws, L.hq), at<float>(ws, L.scale_h), at<unsigned int>(ws, L.arrivals),
+                        at<int32_t>(ws, L.row_expert)};
   bool requant_done = false;
   if ((rc = launch_gateup(at<void>(ws, L.xq), offsets, at<float>(ws, L.scale_x), wg, wu, sg, su, T, D, H, 1,
                           at<void>(ws, L.h), at<float>(ws, L.amax_h), status, at<void>(ws, L.gemm_scratch), st, &fr,

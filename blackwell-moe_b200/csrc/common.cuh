@@ -204,6 +204,7 @@ struct FusedRequant {
   void* hq;
   float* scale_h;
   unsigned int* arrivals;
+  const int32_t* row_expert;      // expert of every permuted row, -1 where no slot owns the row
 };
 int launch_gateup(const void* xq, const int32_t* offsets, const float* sx, const void* wg, const void* wu,
                   const float* sg, const float* su, int M, int D, int H, int E, void* h, float* amax_h,
@@ -222,6 +223,7 @@ struct CombineArgs {
   // permuted row; reduce = add the weighted rows straight into `out` (zeroed by the caller) from the epilogue
   const float* row_w = nullptr;
   const int32_t* row_slot = nullptr;
+  const int32_t* row_expert = nullptr;
   bool reduce = false;
   int n_tail = 0;      // always-on slots at the end of every token's K: added after the scale (see combine_kernel)
 };

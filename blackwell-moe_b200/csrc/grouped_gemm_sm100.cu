@@ -526,7 +526,7 @@ swiglu_from_partials_kernel(const float* __restrict__ partial, int S, int M, int
 constexpr int kFusedItems = 8;
 __global__ void __launch_bounds__(256)
 swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, int M, int H,
-                                    const int32_t* __restrict__ offsets, int E, const float* __restrict__ sx,
+                                    const int32_t* __restrict__ row_expert, const float* __restrict__ sx,
                                     const float* __restrict__ sg, const float* __restrict__ su,
                                     uint8_t* __restrict__ hq, float* __restrict__ seg_amax,
                                     float* __restrict__ scale_h, unsigned int* __restrict__ arrivals,
@@ -534,8 +534,7 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
   chain_wait();
   __shared__ int s_ok;
   const int vec_per_row = H / 4;
-  const int n_rows = min(M, offsets[E]);
-  const long long total = (long long)n_rows * vec_per_row;
+  const long long total = (long long)M * vec_per_row;
   float hv[kFusedItems][4];
   int ex[kFusedItems];
 #pragma unroll
@@ -546,7 +545,7 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
     float amax = 0.f;
     if (item < total) {
     const int m = (int)(item / vec_per_row), v = (int)(item % vec_per_row);
-    const int e = expert_of_row(offsets, E, m);
+    const int e = row_expert[m];             // -1: a row that no slot owns (its expert id was out of range)
     ex[i] = e;
     float g[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
     float4 a[kSplitMax], b[kSplitMax];
@@ -561,7 +560,8 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
       g[0] += a[s].x, g[1] += a[s].y, g[2] += a[s].z, g[3] += a[s].w;
       u[0] += b[s].x, u[1] += b[s].y, u[2] += b[s].z, u[3] += b[s].w;
     }
-    const float inv_g = 1.0f / (sx[e] * sg[e]), inv_u = 1.0f / (sx[e] * su[e]);
+    const int ec = max(e, 0);
+    const float inv_g = 1.0f / (sx[ec] * sg[ec]), inv_u = 1.0f / (sx[ec] * su[ec]);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float gate = bf16_round(g[q] * inv_g);
@@ -569,6 +569,7 @@ swiglu_requant_from_partials_kernel(const float* __restrict__ partial, int S, in
       hv[i][q] = bf16_round(bf16_round(silu_f(gate)) * up);
       amax = fmaxf(amax, fabsf(hv[i][q]));
     }
+    if (e < 0) amax = 0.f;                   // (its slab rows hold no result)
     }
     // one atomic per warp when the whole warp works on one expert (the common case), else per thread: tens of
     // thousands of atomics on one address would serialise for longer than the rest of the kernel takes
@@ -647,27 +648,32 @@ down_from_partials_kernel(const float* __restrict__ partial, int S, int M, int D
       make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 
-// The same sum, followed at once by the weighted combine of the token's K rows: one thread per
-// (token, 4 columns).  Arithmetic and order equal down_from_partials_kernel + the combine kernel
-// (bf16 y, bf16 weight, bf16 product, fp32 sum over k in order, optional scale and residual);
-// y is still written so that the staged view of the workspace stays complete.
-__global__ void __launch_bounds__(256)
+// The same sum, followed at once by the weighted combine of the token's K rows.  Arithmetic and order equal
+// down_from_partials_kernel + the combine kernel (bf16 y, bf16 weight, bf16 product, fp32 sum over k in order, optional
+// scale and residual); y is still written so that the staged view of the workspace stays complete.
+// Bound by latency: a block is 32 column vectors x 8 slots, so that a token's rows are fetched side by side (position,
+// then expert and slabs: two dependent trips, whatever K is) and a single token already spreads over D/128 blocks.  One
+// thread per vector that walked its K rows - each with a bisection of the offsets - took 16.7 us at D=2048, K=8, 66 groups.
+constexpr int kCombineSlots = 8;
+__global__ void __launch_bounds__(32 * kCombineSlots)
 down_combine_from_partials_kernel(const float* __restrict__ partial, int S, int M, int D,
-                                  const int32_t* __restrict__ offsets, int E, const float* __restrict__ sh,
+                                  const int32_t* __restrict__ row_expert, const float* __restrict__ sh,
                                   const float* __restrict__ sd, __nv_bfloat16* __restrict__ y,
-                                  const int32_t* __restrict__ pos, const float* __restrict__ weights, int T, int K,
+                                  const int32_t* __restrict__ pos, const float* __restrict__ weights, int K,
                                   __nv_bfloat16* __restrict__ out, float scale,
                                   const __nv_bfloat16* __restrict__ residual, int n_tail) {
   chain_wait();
-  const int vec_per_row = D / 4;
-  const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (size_t)T * vec_per_row) return;
-  const int t = (int)(gid / vec_per_row), v = (int)(gid % vec_per_row);
-  float acc[4] = {0.f, 0.f, 0.f, 0.f}, tail[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k = 0; k < K; ++k) {
+  __shared__ float4 s_prod[32][32];             // [slot][column vector]: bf16(y * w), held in fp32
+  __shared__ bool s_live[32];
+  const int vec_per_row = D / 4, blocks_per_row = (vec_per_row + 31) / 32;
+  const int t = blockIdx.x / blocks_per_row, lane = threadIdx.x & 31, slot0 = threadIdx.x >> 5;
+  const int v = (blockIdx.x - t * blocks_per_row) * 32 + lane;
+  for (int k = slot0; k < K; k += kCombineSlots) {
     const int m = pos[(size_t)t * K + k];
-    if (m < 0) continue;
-    const int e = expert_of_row(offsets, E, m);
+    const float wk = weights[(size_t)t * K + k];
+    if (lane == 0) s_live[k] = m >= 0;
+    if (m < 0 || v >= vec_per_row) continue;
+    const int e = row_expert[m];
     float a[4] = {0.f, 0.f, 0.f, 0.f};
     float4 q[kSplitMax];
 #pragma unroll
@@ -679,13 +685,18 @@ down_combine_from_partials_kernel(const float* __restrict__ partial, int S, int 
     const __nv_bfloat162 lo = __floats2bfloat162_rn(a[0] * inv, a[1] * inv), hi = __floats2bfloat162_rn(a[2] * inv, a[3] * inv);
     reinterpret_cast<uint2*>(y + (size_t)m * D)[v] =
         make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-    const float w = bf16_round(weights[(size_t)t * K + k]);
+    const float w = bf16_round(wk);
     const float2 f0 = __bfloat1622float2(lo), f1 = __bfloat1622float2(hi);
+    s_prod[k][lane] = make_float4(bf16_round(f0.x * w), bf16_round(f0.y * w), bf16_round(f1.x * w), bf16_round(f1.y * w));
+  }
+  __syncthreads();
+  if (slot0 != 0 || v >= vec_per_row) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, tail[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int k = 0; k < K; ++k) {
+    if (!s_live[k]) continue;
+    const float4 p = s_prod[k][lane];
     float* dst = k < K - n_tail ? acc : tail;          // always-on slots are summed apart (see combine_kernel)
-    dst[0] += bf16_round(f0.x * w);
-    dst[1] += bf16_round(f0.y * w);
-    dst[2] += bf16_round(f1.x * w);
-    dst[3] += bf16_round(f1.y * w);
+    dst[0] += p.x, dst[1] += p.y, dst[2] += p.z, dst[3] += p.w;
   }
   if (scale != 1.0f) {     // bf16 tensor times a Python scalar: fp32 product with the unrounded scalar
 #pragma unroll
@@ -821,12 +832,15 @@ int launch_gateup(const void* xq, const int32_t* offsets, const float* sx, const
   if (int rc = launch_gemm<true, true>(ma, mg, mu, p, M, st)) return rc;
   const size_t n = (size_t)M * (H / 4);
   // small batches inside the whole forward: SwiGLU and the requantisation of h in one kernel (no 16-bit h)
-  // as many blocks as there are SMs (all resident at once: they meet inside the kernel), at most kFusedItems items
-  // per thread
-  const size_t fused_blocks = std::min<size_t>((size_t)sm_count(), (n + 255) / 256);
-  if (fr != nullptr && requant_done != nullptr && n <= fused_blocks * 256 * kFusedItems) {
-    BWMOE_CUDA_OK(launch_chained(swiglu_requant_from_partials_kernel, dim3((unsigned)fused_blocks), dim3(256), 0, st,
-        p.partial, sp.split_k, M, H, offsets, E, sx, sg, su, static_cast<uint8_t*>(fr->hq), amax_h, fr->scale_h,
+  // at most as many blocks as there are SMs (all resident at once: they meet inside the kernel) and kFusedItems items
+  // per thread; the blocks are made smaller while the batch does not fill the chip (two rows of H=14336 on 28 blocks of
+  // 256 threads: 8.9 us, most of it waiting for loads that few SMs have to issue)
+  unsigned threads = 256;
+  while (threads > 64 && (n + threads / 2 - 1) / (threads / 2) <= (size_t)sm_count()) threads /= 2;
+  const size_t fused_blocks = std::min<size_t>((size_t)sm_count(), (n + threads - 1) / threads);
+  if (fr != nullptr && requant_done != nullptr && n <= fused_blocks * threads * kFusedItems) {
+    BWMOE_CUDA_OK(launch_chained(swiglu_requant_from_partials_kernel, dim3((unsigned)fused_blocks), dim3(threads), 0, st,
+        p.partial, sp.split_k, M, H, fr->row_expert, sx, sg, su, static_cast<uint8_t*>(fr->hq), amax_h, fr->scale_h,
         fr->arrivals, status, p.amax_last));
     BWMOE_CUDA_OK(cudaGetLastError());
     *requant_done = true;
@@ -882,11 +896,11 @@ int launch_down(const void* hq, const int32_t* offsets, const float* sh, const v
   BWMOE_REQUIRE(scratch != nullptr && aligned16(scratch), BWMOE_ERR_WORKSPACE, "down: scratch buffer required");
   p.partial = static_cast<float*>(scratch);
   if (int rc = launch_gemm<false, true>(ma, mb, mb, p, M, st)) return rc;
-  if (combine != nullptr && combine_state != nullptr && combine->T * combine->K == M) {
-    const size_t nt = (size_t)combine->T * (D / 4);
-    BWMOE_CUDA_OK(launch_chained(down_combine_from_partials_kernel, dim3((unsigned)((nt + 255) / 256)), dim3(256), 0, st,
-        p.partial, sp.split_k, M, D, offsets, E, sh, sd, static_cast<__nv_bfloat16*>(y), combine->pos,
-        combine->weights, combine->T, combine->K, static_cast<__nv_bfloat16*>(combine->out), combine->scale,
+  if (combine != nullptr && combine_state != nullptr && combine->T * combine->K == M && combine->row_expert != nullptr) {
+    const unsigned blocks = (unsigned)combine->T * (unsigned)ceil_div(D / 4, 32);
+    BWMOE_CUDA_OK(launch_chained(down_combine_from_partials_kernel, dim3(blocks), dim3(32 * kCombineSlots), 0, st,
+        p.partial, sp.split_k, M, D, combine->row_expert, sh, sd, static_cast<__nv_bfloat16*>(y), combine->pos,
+        combine->weights, combine->K, static_cast<__nv_bfloat16*>(combine->out), combine->scale,
         static_cast<const __nv_bfloat16*>(combine->residual), combine->n_tail));
     BWMOE_CUDA_OK(cudaGetLastError());
     *combine_state = kCombineDone;

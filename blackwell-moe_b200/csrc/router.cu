@@ -169,19 +169,23 @@ __device__ void exact_logits_block(const __nv_bfloat16* __restrict__ xrow, const
 // partial logits in its shared memory; after a cluster barrier CTA 0 adds the partials of its peers in
 // rank order (distributed shared memory) and selects.
 // ---------------------------------------------------------------------------------------
-constexpr int kTokenSmemBytes = 32 * 256 * (int)sizeof(double);     // per-warp partial logits
+// Dynamic shared memory: the partial logits of every warp, and (in CTA 0 of a cluster) those of every CTA.  Sized by the
+// experts and warps there are: a fixed 64 KiB left three blocks to an SM, which a batch of a thousand tokens and eight
+// experts noticed (33.8 us).
+inline int token_smem_bytes(int threads, int C, int E) { return (threads / 32 + (C > 1 ? C : 0)) * E * (int)sizeof(double); }
 __global__ void __launch_bounds__(1024)
 router_token_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int T, int D,
                     int E, int K, const RouteRows out, float* __restrict__ row_amax, uint32_t* __restrict__ zero,
                     int zero_words) {
   chain_wait();
-  extern __shared__ __align__(16) double token_part[];          // [nwarps][256]
-  __shared__ double lgd[256];                                   // this CTA's partial logits
+  extern __shared__ __align__(16) double token_part[];          // [nwarps][E], then [C][E]
   __shared__ float lg[256];
   __shared__ float s_max[32];
+  __shared__ float s_cta_max[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  if (C > 1) cluster.barrier_arrive();          // (waited for before the first store into CTA 0's shared memory)
   const int tok = blockIdx.x / C;
   const __nv_bfloat16* xrow = x + (size_t)tok * D;
   // words the later kernels of the call want to find at zero (a memset node of its own costs more than this)
@@ -240,40 +244,45 @@ router_token_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
   }
   if (lane < V && ev_ok) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) token_part[warp * 256 + 8 * ev + j] = acc[j];
+    for (int j = 0; j < 8; ++j) token_part[warp * E + 8 * ev + j] = acc[j];
   }
   for (int off = 16; off; off >>= 1) xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, off));
   if (lane == 0) s_max[warp] = xmax;
   __syncthreads();
-  // warp w sums experts w, w + nwarps, ...; lane l brings warp l's part
-  for (int e = warp; e < E; e += nwarps) {
-    double v = lane < nwarps ? token_part[lane * 256 + e] : 0.0;
-    for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane == 0) lgd[e] = v;
-  }
+  // thread e adds the warps' parts of expert e, in order; the CTAs then put theirs side by side in CTA 0
+  double* cta_part = token_part + nwarps * E;
   if (C > 1) {
-    cluster.sync();
-    if (rank == 0) {
-      for (int e = tid; e < E; e += blockDim.x) {
-        double v = lgd[e];
-        for (int r = 1; r < C; ++r) v += cluster.map_shared_rank(lgd, r)[e];
-        lg[e] = (float)v;                                 // the one rounding to fp32
-      }
-      if (tid < nwarps) {
-        float m = s_max[tid];
-        for (int r = 1; r < C; ++r) m = fmaxf(m, cluster.map_shared_rank(s_max, r)[tid]);
-        s_max[tid] = m;
-      }
+    cluster.barrier_wait();
+    double* dst = cluster.map_shared_rank(cta_part, 0) + rank * E;
+    for (int e = tid; e < E; e += blockDim.x) {
+      double v = 0.0;
+#pragma unroll 8
+      for (int w = 0; w < nwarps; ++w) v += token_part[w * E + e];
+      dst[e] = v;
     }
-    cluster.sync();                     // the peers' shared memory has been read: they may leave
+    if (warp == nwarps - 1) {
+      float m = lane < nwarps ? s_max[lane] : 0.f;
+      for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+      if (lane == 0) cluster.map_shared_rank(s_cta_max, 0)[rank] = m;
+    }
+    cluster.sync();                     // every CTA's stores are visible to CTA 0
     if (rank != 0) return;
+    for (int e = tid; e < E; e += blockDim.x) {
+      double v = 0.0;
+      for (int r = 0; r < C; ++r) v += cta_part[r * E + e];
+      lg[e] = (float)v;                 // the one rounding to fp32
+    }
   } else {
-    __syncthreads();
-    for (int e = tid; e < E; e += blockDim.x) lg[e] = (float)lgd[e];
-    __syncthreads();
+    for (int e = tid; e < E; e += blockDim.x) {
+      double v = 0.0;
+#pragma unroll 8
+      for (int w = 0; w < nwarps; ++w) v += token_part[w * E + e];
+      lg[e] = (float)v;
+    }
   }
+  __syncthreads();
   if (warp == 0) {
-    float m_tok = lane < nwarps ? s_max[lane] : 0.f;
+    float m_tok = C > 1 ? (lane < C ? s_cta_max[lane] : 0.f) : (lane < nwarps ? s_max[lane] : 0.f);
     for (int off = 16; off; off >>= 1) m_tok = fmaxf(m_tok, __shfl_xor_sync(0xffffffffu, m_tok, off));
     select_token(lg, E, K, 0.f, -1.f, out, (size_t)tok, lane);
     if (lane == 0 && row_amax != nullptr) row_amax[tok] = m_tok;
@@ -639,7 +648,7 @@ int launch_router(const void* x, const void* wg, int T, int D, int E, int K, flo
     // Few tokens: a cluster of up to 8 CTAs per token (as many as keep the grid within the SMs), and enough
     // threads that every (expert octet, 8 consecutive d) pair has a thread of its own where that fits.
     static unsigned char smem_set[64] = {0};
-    BWMOE_CUDA_OK(ensure_dynamic_smem(router_token_kernel, kTokenSmemBytes, smem_set));
+    BWMOE_CUDA_OK(ensure_dynamic_smem(router_token_kernel, token_smem_bytes(1024, 8, 256), smem_set));
     int C = 1;
     while (C < 8 && T * C * 2 <= sm_count()) C *= 2;
     int V = 1;
@@ -650,7 +659,7 @@ int launch_router(const void* x, const void* wg, int T, int D, int E, int K, flo
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(T * C));
     cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = kTokenSmemBytes;
+    cfg.dynamicSmemBytes = (size_t)token_smem_bytes(threads, C, E);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
