@@ -705,7 +705,8 @@ inline unsigned quant_grid(int M, int W) { return (unsigned)(((size_t)M * (W / 1
 
 size_t plan_scratch_bytes(int T, int E, int K) {
   const long long M = (long long)T * K;
-  const long long per = plan_slots_per_block(M), B = (M + per - 1) / per;
+  // never less for more slots, although fewer blocks may be used there: a workspace sized for a batch serves smaller ones
+  const long long B = std::min<long long>((M + 2 * kPlanThreads - 1) / (2 * kPlanThreads), kPlanMaxBlocks);
   return (size_t)(B * E * sizeof(int32_t) + 256);
 }
 

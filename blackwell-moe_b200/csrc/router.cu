@@ -165,9 +165,9 @@ __device__ void exact_logits_block(const __nv_bfloat16* __restrict__ xrow, const
 // d-groups spread over the 1-8 CTAs of the cluster so that a few tokens still pull the gate matrix through
 // many SMs at once.  The products (exact in fp32) are accumulated in fp64 - a few thousand DFMAs per SM
 // disappear behind the loads here - so the sums ARE the exact logits, rounded once to fp32: no error
-// bound, no tie detection, no second pass.  Every CTA reduces its own share in a fixed shuffle tree to
-// partial logits in its shared memory; after a cluster barrier CTA 0 adds the partials of its peers in
-// rank order (distributed shared memory) and selects.
+// bound, no tie detection, no second pass.  Every CTA adds up its own share in a fixed order and
+// stores its partial logits into CTA 0's shared memory; after a cluster barrier CTA 0 adds those in rank
+// order and selects.
 // ---------------------------------------------------------------------------------------
 // Dynamic shared memory: the partial logits of every warp, and (in CTA 0 of a cluster) those of every CTA.  Sized by the
 // experts and warps there are: a fixed 64 KiB left three blocks to an SM, which a batch of a thousand tokens and eight

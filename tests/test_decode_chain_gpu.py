@@ -1,0 +1,142 @@
+"""The kernels and dispatch rules of decode-sized calls at the sizes where they can go wrong, against the oracle: the plan
+and quantisation in one launch (up to 1024 slots) and the two-pass plan beyond, split-K post passes (up to 64 rows), the
+block-scale tiles that read back 8, 16 or 32 token columns and share their K blocks among the CTAs of a cluster (up to 8
+rows), always-on experts written by the router, caller-routed batches, and the router's candidate bounds."""
+
+import pytest
+import torch
+
+import oracle
+from helpers import BF16, check_against_oracle, make_inputs, run_cuda_forward, run_oracle_forward, to_cuda
+from test_block_gpu import make_block_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+# rows T*K of 1, 8, 16, 17, 64, 65, 1024 and 1025; ragged D and H; all experts selected; more experts than rows
+@pytest.mark.parametrize("T,D,E,K,H", [(1, 256, 4, 1, 64), (1, 272, 8, 8, 144), (2, 1040, 16, 8, 320), (17, 256, 4, 1, 128),
+                                       (8, 512, 8, 8, 1408), (13, 256, 16, 5, 208), (3, 2048, 66, 8, 1408),
+                                       (1024, 128, 16, 1, 64), (1025, 144, 16, 1, 64), (128, 400, 256, 8, 48)])
+def test_per_tensor_forward_at_the_edges_of_the_dispatch(T, D, E, K, H):
+    inp = make_inputs(T, D, E, K, H, seed=T * 7 + K)
+    out, views = run_cuda_forward(inp)
+    ref, inter = run_oracle_forward(inp)
+    check_against_oracle(inp, out, views, ref, inter)
+
+
+# one token: clusters of 4 (8 tiles of 8 K blocks), of 2 (40 and 64 tiles; 5 K blocks in unequal shares), none (down: 2 K
+# blocks); 8 rows in one expert; 9 rows: no clusters; segments of up to 8, 16 and 32 rows and beyond one 32-row tile
+@pytest.mark.parametrize("T,D,E,K,H", [(1, 1024, 16, 8, 128), (1, 1024, 16, 8, 640), (1, 2048, 128, 8, 768), (1, 640, 8, 3, 384),
+                                       (2, 512, 8, 4, 256), (8, 512, 1, 1, 256), (9, 1024, 2, 1, 256), (24, 384, 8, 2, 576),
+                                       (40, 512, 16, 3, 208), (70, 256, 32, 2, 144), (1024, 128, 256, 1, 128), (1025, 272, 160, 1, 128)])
+def test_block_forward_at_the_edges_of_the_dispatch(T, D, E, K, H):
+    import blackwell_moe_b200 as bw
+    inp = make_block_inputs(T, D, E, K, H, seed=T + D)
+    c = to_cuda(inp)
+    call = lambda: bw.fp8_moe_forward(c["x"], c["w_gate"], c["q_gate"], c["q_up"], c["q_down"],
+                                      c["inv_gate"], c["inv_up"], c["inv_down"], top_k=K)
+    out = call()
+    v = {k: t.cpu() for k, t in bw.moe_stage_views("cuda:0", T, D, H, E, K, block=True).items()}
+    inter = {}
+    ref = oracle.moe_forward_block_recipe(inp["x"], inp["w_gate"], inp["q_gate"], inp["q_up"], inp["q_down"],
+                                          inp["inv_gate"], inp["inv_up"], inp["inv_down"], top_k=K, intermediates=inter)
+    assert int(v["status"][0]) == 0
+    for name, want in (("indices", "indices"), ("offsets", "offsets"), ("x_inv", "x_inv")):
+        assert torch.equal(v[name], inter[want]), name
+    assert torch.equal(v["row_slot"].long(), inter["sort_perm"])
+    assert torch.equal(v["xq"].view(torch.uint8), inter["xq"].view(torch.uint8))
+    assert (v["hq"].view(torch.uint8) != inter["hq"].view(torch.uint8)).float().mean().item() < 0.02
+    assert oracle.rel_l1(v["y"], inter["y_perm"]) < 1e-2
+    assert oracle.rel_l1(out.cpu(), ref) < 1e-2
+    assert torch.equal(call(), out)                     # sums in a fixed order
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 150])           # 8, 64, 72 and 1200 rows: fused and separate requantisation
+def test_always_on_experts_share_one_scale_and_follow_the_routed_slots(T):
+    import blackwell_moe_b200 as bw
+    D, E, K, H, S = 512, 16, 6, 256, 2
+    inp = make_inputs(T, D, E, K, H, seed=T + 3)
+    shared = [oracle.quant_fp8_e4m3((torch.randn(a, b, generator=torch.Generator().manual_seed(i)) * 0.02).to(BF16))
+              for i, (a, b) in enumerate(((D, S * H), (D, S * H), (S * H, D)))]
+    c = to_cuda(inp)
+    stacked = bw.stack_shared_experts(c["q_gate"], c["q_up"], c["q_down"], c["s_gate"], c["s_up"], c["s_down"],
+                                      *[q.cuda() for q, _ in shared], *[s.float().cuda() for _, s in shared])
+    out = bw.fp8_moe_forward_shared(c["x"], c["w_gate"], *stacked[:6], top_k=K, n_shared=S, routed_scale=1.5)
+    routed, _ = run_oracle_forward(inp)
+    sh = oracle.shared_expert_fp8(inp["x"], *[q for q, _ in shared], *[s for _, s in shared])
+    ref = ((routed * 1.5).to(BF16) + sh).to(BF16)
+    assert oracle.rel_l1(out.cpu(), ref) < 1e-2
+
+
+@pytest.mark.parametrize("block", [False, True])
+@pytest.mark.parametrize("T", [1, 37, 700])
+def test_caller_routed_batches_equal_the_routed_forward(T, block):
+    """Ids through a remap table, ids as slots, and the whole forward: the same rows, bit for bit; a missing expert is
+    reported and its slots own no row."""
+    import blackwell_moe_b200 as bw
+    D, E, K, H = 256, 16, 4, 128
+    inp = make_block_inputs(T, D, E, K, H, seed=T) if block else make_inputs(T, D, E, K, H, seed=T)
+    c = to_cuda(inp)
+    s = "inv_" if block else "s_"
+    w = (c["q_gate"], c["q_up"], c["q_down"], c[s + "gate"], c[s + "up"], c[s + "down"])
+    full = bw.fp8_moe_forward(c["x"], c["w_gate"], *w, top_k=K)
+    wt, idx = bw.top_k_router(c["x"], c["w_gate"], K)
+    assert torch.equal(bw.fp8_moe_forward_routed(c["x"], wt, idx, *w), full)
+    ids = torch.randperm(40, generator=torch.Generator().manual_seed(1))[:E].cuda()
+    remap = torch.full((40,), -1, dtype=torch.int32, device="cuda")
+    remap[ids] = torch.arange(E, dtype=torch.int32, device="cuda")
+    named = ids[idx.long()].to(torch.int32)
+    assert torch.equal(bw.fp8_moe_forward_routed(c["x"], wt, named, *w, remap=remap), full)
+    gone = named.clone()
+    gone[0, 1] = next(i for i in range(40) if int(remap[i]) < 0)
+    bw.fp8_moe_forward_routed(c["x"], wt, gone, *w, remap=remap)
+    v = bw.moe_stage_views("cuda:0", T, D, H, E, K, block=block)
+    assert int(v["status"][0]) & 2 and int(v["offsets"][-1]) == T * K - 1 and int(v["pos"].view(T, K)[0, 1]) == -1
+
+
+@pytest.mark.parametrize("M,E", [(1025, 7), (2048, 256), (2049, 64), (70001, 200), (524289, 16), (600000, 256)])
+def test_two_pass_plan_is_the_stable_sort(M, E):
+    from blackwell_moe_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator().manual_seed(M)
+    ids = torch.randint(0, E, (M,), generator=g, dtype=torch.int32)
+    ids[torch.randint(0, M, (5,), generator=g)] = E                     # slots that own no row
+    amax = torch.rand(M, generator=g)
+    i32 = lambda n, fill=-7: torch.full((n,), fill, dtype=torch.int32, device="cuda")
+    offsets, pos, row_slot, row_expert, status = i32(E + 1), i32(M), i32(M), i32(M), i32(1, 0)
+    seg = torch.full((E,), 9.0, device="cuda")
+    scratch = torch.empty(lib.bwmoe_plan_scratch_bytes(M, E, 1), dtype=torch.uint8, device="cuda")
+    d_ids, d_amax = ids.cuda(), amax.cuda()
+    _lib.check(lib.bwmoe_permute_plan(d_ids.data_ptr(), d_amax.data_ptr(), M, E, 1, offsets.data_ptr(), pos.data_ptr(),
+                                      row_slot.data_ptr(), row_expert.data_ptr(), seg.data_ptr(), status.data_ptr(),
+                                      scratch.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    order = torch.sort(ids, stable=True).indices
+    n = int((ids < E).sum())
+    assert int(status[0]) == 2
+    assert torch.equal(offsets.cpu().long(), torch.searchsorted(ids[order], torch.arange(E + 1, dtype=torch.int32)))
+    assert torch.equal(row_slot.cpu().long()[:n], order[:n]) and torch.all(row_slot[n:] == -1)
+    assert torch.equal(row_expert.cpu()[:n], ids[order[:n]]) and torch.all(row_expert[n:] == -1)
+    want = torch.full((M,), -1, dtype=torch.int64)
+    want[order[:n]] = torch.arange(n)
+    assert torch.equal(pos.cpu().long(), want)
+    ref = torch.zeros(E).scatter_reduce(0, ids[order[:n]].long(), amax[order[:n]], "amax")
+    assert torch.equal(seg.cpu(), ref)
+
+
+@pytest.mark.parametrize("T,D,E,K", [(8, 2048, 64, 6), (64, 1024, 256, 8), (300, 2048, 128, 8), (2000, 1024, 256, 8), (1024, 512, 8, 2)])
+def test_router_with_columns_of_very_different_length(T, D, E, K):
+    """Skewed popularity through a constant feature (one column several times as long as the others), tokens of zeros
+    (all logits tie) and a duplicated column: still the exact order, ties to the lower id."""
+    import blackwell_moe_b200 as bw
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, D, generator=g).to(BF16)
+    w = (torch.randn(D, E, generator=g) * 0.02).to(BF16)
+    x[:, 0] = 1.0
+    w[0] = (-1.1 * torch.log(torch.randperm(E, generator=g).float() + 1.0) + 3.0).to(BF16)
+    w[:, E // 2] = w[:, 1]
+    x[T // 2] = 0
+    wt, idx = bw.top_k_router(x.cuda(), w.cuda(), K)
+    wr, ir = oracle.router_canonical(x, w, K)
+    assert torch.equal(idx.cpu(), ir)
+    torch.testing.assert_close(wt.cpu(), wr, rtol=1e-3, atol=1e-4)
