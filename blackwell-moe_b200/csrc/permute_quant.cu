@@ -582,40 +582,41 @@ combine_peers_kernel(const PeerPtrs src, const int32_t* __restrict__ pos, const 
 // n_tail: the last n_tail slots of every token are always-on (shared) experts run as extra groups of the same
 // pipeline; their rows are the `shared` term of the glue above: out = bf16( bf16(routed * scale) + bf16(sum of
 // the tail rows) ).
-template <bool PREWEIGHTED>
+// Bound by memory: a token's K rows are gathered once and its result written once.  A warp serves 32 vectors of ONE token,
+// so lane k fetches the position and weight of slot k for all of them, and the rows' vectors - ROWS of them per lane - are
+// then requested side by side.  (A thread that fetched the positions of three rows before their vectors waited twice per
+// three rows: 4.2 TB/s at 32768 tokens x 8 rows of 2048.)
+template <bool PREWEIGHTED, int ROWS>
 __global__ void __launch_bounds__(256)
 combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ pos,
                const float* __restrict__ weights, int T, int D, int K, __nv_bfloat16* __restrict__ out,
                float scale, const __nv_bfloat16* __restrict__ residual, int n_tail) {
   chain_wait();
-  const int vec_per_row = D / 8;
-  const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (size_t)T * vec_per_row) return;
-  const int t = (int)(gid / vec_per_row), v = (int)(gid % vec_per_row);
+  const int vec_per_row = D / 8, warps_per_row = (vec_per_row + 31) / 32;
+  const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int t = (int)(warp / (unsigned)warps_per_row), lane = threadIdx.x & 31;
+  if (t >= T) return;                               // the whole warp
+  const int v = (int)(warp - (unsigned)t * (unsigned)warps_per_row) * 32 + lane;
+  const bool v_ok = v < vec_per_row;
+  const int my_pos = lane < K ? pos[(size_t)t * K + lane] : -1;
+  const float my_w = (!PREWEIGHTED && lane < K) ? bf16_round(weights[(size_t)t * K + lane]) : 0.f;
   const int k_routed = K - n_tail;
   float acc[8], tail[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f, tail[i] = 0.f;
-  // three rows at a time: their vectors are all requested before the first is used (one load in flight
-  // per thread left the gather at 5.2 TB/s; eight cost too many registers)
-  constexpr int kRows = 3;
-  for (int k0 = 0; k0 < K; k0 += kRows) {
-    int p[kRows];
-    float w[kRows];
-    uint4 raw[kRows];
+  for (int k0 = 0; k0 < K; k0 += ROWS) {
+    int p[ROWS];
+    uint4 raw[ROWS];
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
-      const bool in_k = k0 + j < K;
-      p[j] = in_k ? pos[(size_t)t * K + k0 + j] : -1;
-      w[j] = (in_k && !PREWEIGHTED) ? weights[(size_t)t * K + k0 + j] : 0.f;
+    for (int j = 0; j < ROWS; ++j) {
+      p[j] = __shfl_sync(0xffffffffu, my_pos, (k0 + j) & 31);
+      if (k0 + j >= K) p[j] = -1;
+      raw[j] = p[j] >= 0 && v_ok ? __ldcs(reinterpret_cast<const uint4*>(y + (size_t)p[j] * D) + v) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
-    for (int j = 0; j < kRows; ++j)
-      raw[j] = p[j] >= 0 ? reinterpret_cast<const uint4*>(y + (size_t)p[j] * D)[v] : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-    for (int j = 0; j < kRows; ++j) {
-      if (p[j] < 0) continue;
-      const float wk = bf16_round(w[j]);
+    for (int j = 0; j < ROWS; ++j) {
+      const float wk = PREWEIGHTED ? 0.f : __shfl_sync(0xffffffffu, my_w, (k0 + j) & 31);
+      if (p[j] < 0) continue;                       // (the same in every lane)
       const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -626,6 +627,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ 
       }
     }
   }
+  if (!v_ok) return;
   if (scale != 1.0f) {     // bf16 tensor times a Python scalar: torch multiplies in fp32 by the unrounded scalar
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = bf16_round(bf16_round(acc[i]) * scale);
@@ -899,15 +901,15 @@ int launch_combine(const void* y, const int32_t* pos, const float* weights, int 
   BWMOE_REQUIRE(T > 0 && D > 0 && K > 0 && D % 8 == 0, BWMOE_ERR_BAD_SHAPE, "combine: T=%d D=%d K=%d", T, D, K);
   BWMOE_REQUIRE(y && pos && weights && out, BWMOE_ERR_NULL, "combine: null pointer");
   BWMOE_REQUIRE(aligned16(y) && aligned16(out), BWMOE_ERR_BAD_ALIGN, "combine: pointers must be 16-byte aligned");
-  const size_t n = (size_t)T * (D / 8);
-  if (preweighted)
-    BWMOE_CUDA_OK(launch_chained(combine_kernel<true>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st,
-        static_cast<const __nv_bfloat16*>(y), pos, weights, T, D, K, static_cast<__nv_bfloat16*>(out), scale,
-        static_cast<const __nv_bfloat16*>(residual), n_tail));
-  else
-    BWMOE_CUDA_OK(launch_chained(combine_kernel<false>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st,
-        static_cast<const __nv_bfloat16*>(y), pos, weights, T, D, K, static_cast<__nv_bfloat16*>(out), scale,
-        static_cast<const __nv_bfloat16*>(residual), n_tail));
+  const size_t warps = (size_t)T * ceil_div(D / 8, 32);
+  const dim3 grid((unsigned)((warps + 7) / 8)), block(256);
+  auto launch = [&](auto kernel) {
+    return launch_chained(kernel, grid, block, 0, st, static_cast<const __nv_bfloat16*>(y), pos, weights, T, D, K,
+                          static_cast<__nv_bfloat16*>(out), scale, static_cast<const __nv_bfloat16*>(residual), n_tail);
+  };
+  // as many rows in flight as a token has, eight at most (their registers then cost occupancy)
+  if (preweighted) BWMOE_CUDA_OK(K <= 2 ? launch(combine_kernel<true, 2>) : K <= 4 ? launch(combine_kernel<true, 4>) : launch(combine_kernel<true, 8>));
+  else             BWMOE_CUDA_OK(K <= 2 ? launch(combine_kernel<false, 2>) : K <= 4 ? launch(combine_kernel<false, 4>) : launch(combine_kernel<false, 8>));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }
