@@ -95,7 +95,7 @@ inline size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 // Workspace layout.  The first block (status .. amax_h) is cleared by one memset per call.
 struct Layout {
-  size_t status, amax_x, amax_h, arrivals, zero_end;
+  size_t status, amax_x, amax_h, arrivals, router_head, zero_end;
   size_t offsets, scale_x, scale_h, topk_idx, topk_w, row_amax, pos, row_slot, row_expert, row_w;
   size_t plan_scratch, gemm_scratch, router_scratch, router_scratch_bytes, xq, h, hq, y, total;
 };
@@ -115,6 +115,7 @@ bool make_layout(int T, int D, int H, int E, int K, Layout* L, int n_shared = 0)
   L->amax_x = take(sizeof(float) * E);
   L->amax_h = take(sizeof(float) * E);
   L->arrivals = take(16);
+  L->router_head = take(kRouterHeadBytes);
   L->zero_end = o;
   L->offsets = take(sizeof(int32_t) * (E + 1));
   L->scale_x = take(sizeof(float) * E);
@@ -141,7 +142,7 @@ bool make_layout(int T, int D, int H, int E, int K, Layout* L, int n_shared = 0)
 
 // Workspace of the block-scale recipe: no bf16 h, no segment statistics; per-row group scales instead.
 struct BlockLayout {
-  size_t status, zero_end, offsets, topk_idx, topk_w, row_amax, pos, row_slot, row_expert, plan_scratch;
+  size_t status, router_head, zero_end, offsets, topk_idx, topk_w, row_amax, pos, row_slot, row_expert, plan_scratch;
   size_t router_scratch, router_scratch_bytes, xq, x_inv, hq, h_inv, y, total;
 };
 
@@ -156,6 +157,7 @@ bool make_block_layout(int T, int D, int H, int E, int K, BlockLayout* L) {
     return at;
   };
   L->status = take(16);
+  L->router_head = take(kRouterHeadBytes);
   L->zero_end = o;
   L->offsets = take(sizeof(int32_t) * (E + 1));
   L->topk_idx = take(sizeof(int32_t) * M);
@@ -431,7 +433,7 @@ int bwmoe_moe_forward(const void* x, const void* w_gate, const void* wg, const v
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end, at<void>(ws, L.router_head)))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st);
 }
@@ -449,7 +451,7 @@ int bwmoe_moe_forward_flags(const void* x, const void* w_gate, const void* wg, c
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end, at<void>(ws, L.router_head)))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st, 1.0f, nullptr,
                       flags);
@@ -471,7 +473,7 @@ int bwmoe_moe_forward_shared(const void* x, const void* w_gate, const void* wg, 
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, S, ws, L.zero_end))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, S, ws, L.zero_end, at<void>(ws, L.router_head)))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E + S, K + S, out, ws, L, st,
                       routed_scale, nullptr, 0, S);
@@ -491,7 +493,7 @@ int bwmoe_moe_forward_ex(const void* x, const void* w_gate, const void* wg, cons
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   float* row_amax = at<float>(ws, L.row_amax);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, row_amax, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end, at<void>(ws, L.router_head)))
     return rc;
   return run_pipeline(x, weights, indices, row_amax, wg, wu, wd, sg, su, sd, T, D, H, E, K, out, ws, L, st,
                       routed_scale, residual);
@@ -633,7 +635,7 @@ int bwmoe_moe_forward_block(const void* x, const void* w_gate, const void* wg, c
   float* weights = at<float>(ws, L.topk_w);
   int32_t* indices = at<int32_t>(ws, L.topk_idx);
   if (int rc = launch_router(x, w_gate, T, D, E, K, weights, indices, nullptr, st, at<void>(ws, L.router_scratch),
-                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end))
+                             L.router_scratch_bytes, at<int32_t>(ws, L.status), 0, 0, ws, L.zero_end, at<void>(ws, L.router_head)))
     return rc;
   return run_block_pipeline(x, weights, indices, wg, wu, wd, inv_g, inv_u, inv_d, T, D, H, E, K, out, ws, L, st);
 }

@@ -138,18 +138,21 @@ struct RouteRows {
 // scratch (optional): enables the tensor-core router where it applies; needs router_scratch_bytes()
 // n_tail: always-on slots appended to every token's K (see RouteRows; weights / indices are [T, K + n_tail]).
 // zero: words to be cleared before any later kernel of the stream runs (and before `status` can be raised).
+// zeroed_head: kRouterHeadBytes of them for the router's own use (one memset node instead of two).
 // T_as > 0: choose the routing kernel a batch of T_as tokens would get (the kernels agree on the selected
 // experts always, but their fp32 weights differ in the last bits: a rank that routes a slice of a larger batch
 // passes the size of the whole batch to obtain the weights the whole batch would have got).
+constexpr size_t kRouterHeadBytes = 260 * sizeof(float);
 size_t router_scratch_bytes(int T, int D, int E, int K, int T_as = 0);
 int launch_router(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
                   int32_t* indices, float* row_amax, cudaStream_t st, void* scratch = nullptr,
                   size_t scratch_bytes = 0, int32_t* status = nullptr, int T_as = 0, int n_tail = 0,
-                  void* zero = nullptr, size_t zero_bytes = 0);
+                  void* zero = nullptr, size_t zero_bytes = 0, void* zeroed_head = nullptr);
 bool router_tc_applicable(int T, int D, int E, int K);
 size_t router_tc_scratch_bytes(int T, int D, int E);
 int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
-                     float* row_amax, int32_t* status, void* scratch, cudaStream_t st);
+                     float* row_amax, int32_t* status, void* scratch, int T_as, void* zeroed_head,
+                     cudaStream_t st);
 int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
                            const int32_t* list, const int32_t* count, cudaStream_t st);
 size_t plan_scratch_bytes(int T, int E, int K);

@@ -621,7 +621,7 @@ size_t router_scratch_bytes(int T, int D, int E, int K, int T_as) {
 
 int launch_router(const void* x, const void* wg, int T, int D, int E, int K, float* weights,
                   int32_t* indices, float* row_amax, cudaStream_t st, void* scratch, size_t scratch_bytes,
-                  int32_t* status, int T_as, int n_tail, void* zero, size_t zero_bytes) {
+                  int32_t* status, int T_as, int n_tail, void* zero, size_t zero_bytes, void* zeroed_head) {
   const int Tc = T_as > 0 ? T_as : T;       // the batch size that picks the kernel (launch sizes follow T)
   BWMOE_REQUIRE(T > 0 && D > 0 && E > 0 && K > 0, BWMOE_ERR_BAD_SHAPE, "router: T=%d D=%d E=%d K=%d", T, D, E, K);
   BWMOE_REQUIRE(E <= 256, BWMOE_ERR_UNSUPPORTED, "router: E=%d > 256", E);
@@ -632,7 +632,7 @@ int launch_router(const void* x, const void* wg, int T, int D, int E, int K, flo
   if (router_tc_applicable(Tc, D, E, K) && scratch != nullptr && scratch_bytes >= router_tc_scratch_bytes(T, D, E) &&
       aligned16(x) && aligned16(wg)) {
     if (zero_bytes > 0) BWMOE_CUDA_OK(cudaMemsetAsync(zero, 0, zero_bytes, st));
-    return launch_router_tc(x, wg, T, D, E, K, out, row_amax, status, scratch, st);
+    return launch_router_tc(x, wg, T, D, E, K, out, row_amax, status, scratch, Tc, zeroed_head, st);
   }
   int Epad = 8;
   while (Epad < E) Epad <<= 1;
@@ -655,7 +655,7 @@ int launch_router(const void* x, const void* wg, int T, int D, int E, int K, flo
     while (V < E / 8) V <<= 1;
     int threads = 256;
     while (threads < 1024 && (long long)threads * C < (long long)V * ceil_div(D, 8)) threads *= 2;
-    if (T > 64 && E < 128) threads = 256;
+    if (T > 64 && E < 128) threads = T > 3 * sm_count() && E <= 16 ? 128 : 256;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(T * C));
     cfg.blockDim = dim3((unsigned)threads);

@@ -63,10 +63,11 @@ transpose_gate_kernel(const __nv_bfloat16* __restrict__ wg, int D, int E, __nv_b
 
 // ---- 2. tensor-core logits + per-token candidate list ------------------------------------
 struct TcParams {
-  float* logits;        // [T, n_mma] fp32
+  float* logits;        // [k_parts, T, n_mma] fp32
   int32_t* status;
   int T, D, E, n_chunks, n_mma;   // n_chunks = ceil(E/64) weight boxes; n_mma = MMA N (multiple of 16)
   int split_n;                    // 1: a work item is (row tile, one 64-expert chunk) - few row tiles, many SMs
+  int k_parts;                    // a work item covers 1/k_parts of the K blocks; refine_kernel adds the parts in order
 };
 
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -122,11 +123,13 @@ tc_logits_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  const int total_tiles = ((p.T + BM - 1) / BM) * (p.split_n ? p.n_chunks : 1);      // work items
-  const int k_blocks = (p.D + R_BK - 1) / R_BK;
+  const int total_tiles = ((p.T + BM - 1) / BM) * (p.split_n ? p.n_chunks : 1) * p.k_parts;      // work items
+  const int all_k_blocks = (p.D + R_BK - 1) / R_BK;
   const uint32_t stage_tx = R_A_BYTES + chunks_per_item * R_BCHUNK_BYTES;
-  // item -> (row tile, first expert chunk, experts of the item rounded up to the MMA's N granularity)
-  auto item_of = [&](int item, int& tile, int& c0, int& n_cols) {
+  // item -> (row tile, first expert chunk, experts of the item rounded up to the MMA's N granularity, part of the K blocks)
+  auto item_of = [&](int item, int& tile, int& c0, int& n_cols, int& part) {
+    part = item % p.k_parts;
+    item /= p.k_parts;
     tile = p.split_n ? item / p.n_chunks : item;
     c0 = p.split_n ? item % p.n_chunks : 0;
     n_cols = p.split_n ? min(64, p.n_mma - 64 * c0) : p.n_mma;
@@ -139,9 +142,10 @@ tc_logits_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int item = blockIdx.x; ok && item < total_tiles; item += gridDim.x) {
-        int tile, c0, n_cols;
-        item_of(item, tile, c0, n_cols);
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        int tile, c0, n_cols, part;
+        item_of(item, tile, c0, n_cols, part);
+        const int kb0 = part * all_k_blocks / p.k_parts, kb1 = (part + 1) * all_k_blocks / p.k_parts;
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!(ok = mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, p.status))) break;
           const uint32_t sa = tiles_base + stage * stage_bytes;
           const uint32_t full = bar_full + 8 * stage;
@@ -159,21 +163,22 @@ tc_logits_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       uint32_t stage = 0, phase = 0, local = 0;
       bool ok = true;
       for (int item = blockIdx.x; ok && item < total_tiles; item += gridDim.x, ++local) {
-        int tile, c0, n_cols;
-        item_of(item, tile, c0, n_cols);
+        int tile, c0, n_cols, part;
+        item_of(item, tile, c0, n_cols, part);
+        const int kb0 = part * all_k_blocks / p.k_parts, kb1 = (part + 1) * all_k_blocks / p.k_parts;
         const uint32_t idesc = idesc0 | ((uint32_t)(n_cols >> 3) << 17);
         const uint32_t buf = local & 1u, use = local >> 1;
         if (!(ok = mbar_wait(bar_tempty + 8 * buf, (use & 1u) ^ 1u, abort_flag, p.status))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!(ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status))) break;
           tc_fence_after();
           const uint32_t sa = tiles_base + stage * stage_bytes;
           const uint64_t da = desc_kmajor(sa), db = desc_nmajor_bf16(sa + R_A_BYTES);
 #pragma unroll
           for (int k = 0; k < R_BK / 16; ++k)   // A: +32 bytes per 16 K; B: +16 K rows = 2048 bytes
-            mma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 128), idesc, (kb | k) != 0 ? 1u : 0u);
+            mma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 128), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           mma_commit(bar_empty + 8 * stage);
           if (++stage == n_stages) stage = 0, phase ^= 1u;
         }
@@ -187,8 +192,8 @@ tc_logits_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     uint32_t local = 0;
     bool ok = true;
     for (int item = blockIdx.x; ok && item < total_tiles; item += gridDim.x, ++local) {
-      int tile, c0, n_cols;
-      item_of(item, tile, c0, n_cols);
+      int tile, c0, n_cols, part;
+      item_of(item, tile, c0, n_cols, part);
       const uint32_t buf = local & 1u, use = local >> 1;
       ok = mbar_wait(bar_tfull + 8 * buf, use & 1u, abort_flag, p.status);
       ok = __all_sync(0xffffffffu, ok);
@@ -196,7 +201,7 @@ tc_logits_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * 256;
       const int row = tile * BM + r_in_tile;
-      float* dst = p.logits + (size_t)row * p.n_mma + c0 * 64;
+      float* dst = p.logits + ((size_t)part * p.T + row) * p.n_mma + c0 * 64;
       for (int c = 0; c < n_cols; c += 32) {
         uint32_t r[32];
         tmem_ld32(t_row + c, r);
@@ -234,7 +239,7 @@ __device__ __forceinline__ void kahan_add_r(float& sum, float& comp, float y) {
 template <int EJ>   // 32 * EJ >= E: logits each lane holds
 __global__ void __launch_bounds__(256)
 refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wgt,
-              const float* __restrict__ wnorm2, const float* __restrict__ logits, int ld_logits, int T, int D,
+              const float* __restrict__ wnorm2, const float* __restrict__ logits, int ld_logits, int k_parts, int T, int D,
               int E, int K, const RouteRows out, float* __restrict__ row_amax,
               int32_t* __restrict__ fallback_count, int32_t* __restrict__ fallback_list) {
   chain_wait();
@@ -278,7 +283,11 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 #pragma unroll
   for (int j = 0; j < EJ; ++j) {
     const int e = lane + 32 * j;
-    key[j] = e < E ? order_key(logits[(size_t)tok * ld_logits + e]) : 0u;      // 0: below every float's key
+    const float* at = logits + (size_t)tok * ld_logits + e;
+    const size_t part = (size_t)T * ld_logits;
+    float v = 0.f;
+    if (e < E) v = k_parts == 1 ? at[0] : (at[0] + at[part]) + (at[2 * part] + at[3 * part]);
+    key[j] = e < E ? order_key(v) : 0u;                  // 0: below every float's key
   }
   float cv = -INFINITY;
   int ci = 0x7fffffff;
@@ -347,6 +356,7 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       const int c = __ffs(rm) - 1;
       const __nv_bfloat16* wrow = wgt + (size_t)__shfl_sync(0xffffffffu, ci, c) * D;
       float acc = 0.f, comp = 0.f;
+#pragma unroll 2
       for (int d0 = lane * 8; d0 < D; d0 += 512) {             // two 8-product steps = one plain-FMA block
         const bool two = d0 + 256 < D;
         const uint4 x0 = *reinterpret_cast<const uint4*>(xrow + d0);
@@ -434,6 +444,14 @@ int make_map_bf16(CUtensorMap* map, const void* base, int rows, int cols, int bo
 struct TcScratch {
   size_t wgt, wnorm2, logits, fb_count, fb_list, total;
 };
+// Few row tiles leave most SMs idle, and each item then waits for its K blocks in a row (32 blocks of 64 at D=2048: 12 us
+// for 128 tokens, 14 us for 4096): the K blocks are split four ways while that still leaves one item per SM and eight
+// blocks per item.  `T_as`, not the number of tokens at hand, decides (the parts' sum rounds differently, and a slice of a
+// batch must get the weights the whole batch would get).
+constexpr int R_K_PARTS = 4;
+int tc_split_rows(int D, int E) { return D >= R_K_PARTS * 8 * R_BK ? 148 / R_K_PARTS / ceil_div(E, 64) * BM : 0; }   // batches up to this
+int tc_k_parts(int T_as, int D, int E) { return T_as <= tc_split_rows(D, E) ? R_K_PARTS : 1; }
+// (sized so that a batch never needs less scratch than a smaller one)
 TcScratch tc_layout(int T, int D, int E) {
   TcScratch s;
   size_t o = 0;
@@ -445,7 +463,7 @@ TcScratch tc_layout(int T, int D, int E) {
   s.wnorm2 = take(sizeof(float) * E);
   s.fb_count = take(sizeof(int32_t) * 4);
   s.wgt = take((size_t)E * D * 2);
-  s.logits = take(sizeof(float) * (size_t)T * (size_t)((E + 15) / 16 * 16));
+  s.logits = take(sizeof(float) * (size_t)std::max(T, R_K_PARTS * std::min(T, tc_split_rows(D, E))) * (size_t)((E + 15) / 16 * 16));
   s.fb_list = take(sizeof(int32_t) * (size_t)T);
   s.total = o;
   return s;
@@ -466,9 +484,11 @@ int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, i
                            const int32_t* list, const int32_t* count, cudaStream_t st);
 
 int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
-                     float* row_amax, int32_t* status, void* scratch, cudaStream_t st) {
+                     float* row_amax, int32_t* status, void* scratch, int T_as, void* zeroed_head,
+                     cudaStream_t st) {
   BWMOE_REQUIRE(scratch != nullptr && aligned16(scratch), BWMOE_ERR_WORKSPACE, "router: scratch buffer required");
   BWMOE_REQUIRE(aligned16(x) && aligned16(wg), BWMOE_ERR_BAD_ALIGN, "router: pointers must be 16-byte aligned");
+  const int k_parts = tc_k_parts(T_as, D, E);
   const TcScratch L = tc_layout(T, D, E);
   uint8_t* base = static_cast<uint8_t*>(scratch);
   auto* wgt = reinterpret_cast<__nv_bfloat16*>(base + L.wgt);
@@ -476,17 +496,23 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
   auto* logits = reinterpret_cast<float*>(base + L.logits);
   auto* fb_count = reinterpret_cast<int32_t*>(base + L.fb_count);
   auto* fb_list = reinterpret_cast<int32_t*>(base + L.fb_list);
-  BWMOE_CUDA_OK(cudaMemsetAsync(base, 0, L.wgt, st));        // column norms, fallback counter, private status word
+  // column norms, fallback counter, private status word: in the caller's cleared block where it has one, else cleared here
+  if (zeroed_head != nullptr) {
+    wnorm2 = static_cast<float*>(zeroed_head);
+    fb_count = static_cast<int32_t*>(zeroed_head) + 256;
+  } else {
+    BWMOE_CUDA_OK(cudaMemsetAsync(base, 0, L.wgt, st));
+  }
   if (status == nullptr) status = fb_count + 1;
   CUtensorMap mx, mw;
   if (int rc = make_map_bf16(&mx, x, T, D, R_BK, BM)) return rc;
   if (int rc = make_map_bf16(&mw, wg, D, E, 64, R_BK)) return rc;
   static unsigned char smem_set[64] = {0};
   BWMOE_CUDA_OK(ensure_dynamic_smem(tc_logits_kernel, R_SMEM_BYTES, smem_set));
-  TcParams p{logits, status, T, D, E, ceil_div(E, 64), ceil_div(E, 16) * 16, 0};
+  TcParams p{logits, status, T, D, E, ceil_div(E, 64), ceil_div(E, 16) * 16, 0, k_parts};
   // few row tiles: one 64-expert chunk per CTA, so that a small batch is spread over several SMs
   p.split_n = (p.n_chunks > 1 && ceil_div(T, BM) * p.n_chunks * 2 <= sm_count()) ? 1 : 0;
-  const int grid = std::min(sm_count(), ceil_div(T, BM) * (p.split_n ? p.n_chunks : 1));
+  const int grid = std::min(sm_count(), ceil_div(T, BM) * (p.split_n ? p.n_chunks : 1) * k_parts);
   BWMOE_CUDA_OK(launch_chained(tc_logits_kernel, dim3(grid), dim3(NUM_THREADS), R_SMEM_BYTES, st, mx, mw, p));
   BWMOE_CUDA_OK(cudaGetLastError());
   BWMOE_CUDA_OK(launch_chained(transpose_gate_kernel, dim3(ceil_div(D, 32), ceil_div(E, 32)), dim3(256), 0, st,
@@ -495,16 +521,16 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
   auto xb = static_cast<const __nv_bfloat16*>(x);
   const unsigned rgrid = (unsigned)ceil_div(T, 8);
   if (E <= 32)
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<1>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<1>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, k_parts, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   else if (E <= 64)
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<2>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<2>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, k_parts, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   else if (E <= 128)
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<4>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<4>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, k_parts, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   else
-    BWMOE_CUDA_OK(launch_chained(refine_kernel<8>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, T, D, E, K, out, row_amax,
+    BWMOE_CUDA_OK(launch_chained(refine_kernel<8>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, k_parts, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   BWMOE_CUDA_OK(cudaGetLastError());
   return launch_router_fallback(x, wg, T, D, E, K, out, fb_list, fb_count, st);
