@@ -585,7 +585,7 @@ combine_peers_kernel(const PeerPtrs src, const int32_t* __restrict__ pos, const 
 // Bound by memory: a token's K rows are gathered once and its result written once.  A warp serves 32 vectors of ONE token,
 // so lane k fetches the position and weight of slot k for all of them, and the rows' vectors - ROWS of them per lane - are
 // then requested side by side.  (A thread that fetched the positions of three rows before their vectors waited twice per
-// three rows: 282 us at 32768 tokens x 8 rows of 2048, 253 now; 104 and 85 us at 16384 x 2 rows of 4096.)
+// three rows: 282 us at 32768 tokens x 8 rows of 2048, 243 now; 104 and 85 us at 16384 x 2 rows of 4096.)
 template <bool PREWEIGHTED, int ROWS>
 __global__ void __launch_bounds__(256)
 combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ pos,
@@ -620,10 +620,10 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ 
       const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float2 f = __bfloat1622float2(q[i]);
-        const float a = PREWEIGHTED ? f.x : bf16_round(f.x * wk), b = PREWEIGHTED ? f.y : bf16_round(f.y * wk);
-        if (k0 + j < k_routed) acc[2 * i] += a, acc[2 * i + 1] += b;
-        else                   tail[2 * i] += a, tail[2 * i + 1] += b;
+        float2 f = __bfloat1622float2(q[i]);
+        if (!PREWEIGHTED) f = __bfloat1622float2(__floats2bfloat162_rn(f.x * wk, f.y * wk));
+        if (k0 + j < k_routed) acc[2 * i] += f.x, acc[2 * i + 1] += f.y;
+        else                   tail[2 * i] += f.x, tail[2 * i + 1] += f.y;
       }
     }
   }
