@@ -140,3 +140,28 @@ def test_router_with_columns_of_very_different_length(T, D, E, K):
     wr, ir = oracle.router_canonical(x, w, K)
     assert torch.equal(idx.cpu(), ir)
     torch.testing.assert_close(wt.cpu(), wr, rtol=1e-3, atol=1e-4)
+
+
+@pytest.mark.parametrize("T,E,block", [(1, 16, False), (40, 16, False), (1, 16, True), (100, 64, True), (600, 64, False)])
+def test_calls_can_be_captured_and_replayed(T, E, block):
+    """The launch chain (cluster launches, programmatic edges, a memset only where the tensor-core router runs) in a CUDA
+    graph: a replay on new activations equals the plain call."""
+    import blackwell_moe_b200 as bw
+    D, K, H = 512, 4, 256
+    inp = make_block_inputs(T, D, E, K, H, seed=T) if block else make_inputs(T, D, E, K, H, seed=T)
+    c = to_cuda(inp)
+    s = "inv_" if block else "s_"
+    w = (c["w_gate"], c["q_gate"], c["q_up"], c["q_down"], c[s + "gate"], c[s + "up"], c[s + "down"])
+    x = c["x"].clone()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        bw.fp8_moe_forward(x, *w, top_k=K)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = bw.fp8_moe_forward(x, *w, top_k=K)
+    x.copy_(c["x"].flip(0))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, bw.fp8_moe_forward(c["x"].flip(0).contiguous(), *w, top_k=K))
