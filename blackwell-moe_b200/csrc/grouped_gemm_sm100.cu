@@ -721,19 +721,24 @@ down_combine_from_partials_kernel(const float* __restrict__ partial, int S, int 
       make_uint2(*reinterpret_cast<const uint32_t*>(&o0), *reinterpret_cast<const uint32_t*>(&o1));
 }
 
-// Split-K is for small batches, where a few experts x column blocks cannot occupy every SM:
-// the K loop of each tile is cut so that about four waves of tiles exist.
+// Split-K is for small batches, where a few experts x column blocks cannot occupy every SM (fewer than four rounds of
+// tiles).  The K loop of each tile is cut into the number of pieces that makes the longest CTA shortest - rounds of pieces
+// x K blocks of a piece - with one per cent per piece for the slabs: two experts of the Mixtral shape (224 gate/up tiles of
+// 32 blocks) take 13 rounds of 4 blocks instead of 5 of 11 (56 -> 53 us), eight of the DeepSeek shape 5 of 2 instead of 4 of 3.
 struct SplitPlan {
   int split_k, k_per_split;
 };
 SplitPlan choose_split(int M, int E, int k_blocks, int n_tiles) {
   SplitPlan sp{1, k_blocks};
-  if (M > kSplitMaxRows) return sp;
   const long long tiles = (long long)std::min(M, E) * n_tiles;      // one row tile per active expert, at most
-  int S = (int)std::min<long long>(kSplitMax, (4ll * sm_count() + tiles - 1) / tiles);
-  S = std::max(1, std::min(S, k_blocks / 2));
-  sp.k_per_split = ceil_div(k_blocks, S);
-  sp.split_k = ceil_div(k_blocks, sp.k_per_split);
+  if (M > kSplitMaxRows || tiles >= 4ll * sm_count()) return sp;
+  double best = 0.0;
+  for (int n = 2; n <= std::min(kSplitMax, k_blocks / 2); ++n) {
+    const int per = ceil_div(k_blocks, n), pieces = ceil_div(k_blocks, per);
+    const long long rounds = (tiles * pieces + sm_count() - 1) / sm_count();
+    const double cost = (double)(rounds * per) * (1.0 + 0.01 * pieces);
+    if (best == 0.0 || cost < best) best = cost, sp = SplitPlan{pieces, per};
+  }
   return sp;
 }
 
