@@ -598,13 +598,18 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ 
   if (t >= T) return;                               // the whole warp
   const int v = (int)(warp - (unsigned)t * (unsigned)warps_per_row) * 32 + lane;
   const bool v_ok = v < vec_per_row;
-  const int my_pos = lane < K ? pos[(size_t)t * K + lane] : -1;
-  const float my_w = (!PREWEIGHTED && lane < K) ? bf16_round(weights[(size_t)t * K + lane]) : 0.f;
+  int my_pos = -1;
+  float my_w = 0.f;
   const int k_routed = K - n_tail;
   float acc[8], tail[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f, tail[i] = 0.f;
   for (int k0 = 0; k0 < K; k0 += ROWS) {
+    if ((k0 & 31) == 0) {                           // 32 slots at a time (a forward has no more; ROWS divides 32)
+      const size_t at = (size_t)t * K + k0 + lane;
+      my_pos = k0 + lane < K ? pos[at] : -1;
+      if (!PREWEIGHTED) my_w = k0 + lane < K ? bf16_round(weights[at]) : 0.f;
+    }
     int p[ROWS];
     uint4 raw[ROWS];
 #pragma unroll

@@ -142,6 +142,30 @@ def test_router_with_columns_of_very_different_length(T, D, E, K):
     torch.testing.assert_close(wt.cpu(), wr, rtol=1e-3, atol=1e-4)
 
 
+@pytest.mark.parametrize("T,D,K", [(1, 8, 1), (5, 264, 2), (3, 256, 5), (7, 1032, 8), (4, 512, 32), (3, 72, 33), (2, 128, 70)])
+def test_combine_stage_with_ragged_rows_and_any_number_of_slots(T, D, K):
+    """The combine entry point: row widths that leave lanes idle, up to 2, 4 and 8 rows in flight, more slots than a warp
+    has lanes, slots without a row - the fixed-order fp32 sum of bf16 products, bit for bit."""
+    from blackwell_moe_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator().manual_seed(T * K)
+    M = T * K
+    y = torch.randn(M, D, generator=g).to(BF16)
+    w = torch.rand(T, K, generator=g)
+    pos = torch.randperm(M, generator=g).to(torch.int32).view(T, K)
+    if K > 2:
+        pos[T - 1, 1] = -1
+    want = torch.zeros(T, D)
+    for k in range(K):
+        prod = (y[pos[:, k].clamp(min=0).long()].float() * w[:, k:k + 1].to(BF16).float()).to(BF16).float()
+        want += torch.where(pos[:, k:k + 1] >= 0, prod, torch.zeros(()))
+    out = torch.empty(T, D, dtype=BF16, device="cuda")
+    d = [t.cuda() for t in (y, pos, w)]
+    _lib.check(lib.bwmoe_combine(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), T, D, K, out.data_ptr(),
+                                 torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(out.cpu(), want.to(BF16))
+
+
 @pytest.mark.parametrize("T,E,block", [(1, 16, False), (40, 16, False), (1, 16, True), (100, 64, True), (600, 64, False)])
 def test_calls_can_be_captured_and_replayed(T, E, block):
     """The launch chain (cluster launches, programmatic edges, a memset only where the tensor-core router runs) in a CUDA
