@@ -447,10 +447,12 @@ struct TcScratch {
 // Few row tiles leave most SMs idle, and each item then waits for its K blocks in a row (32 blocks of 64 at D=2048: 12 us
 // for 128 tokens, 14 us for 4096): the K blocks are split four ways while that still leaves one item per SM and eight
 // blocks per item.  `T_as`, not the number of tokens at hand, decides (the parts' sum rounds differently, and a slice of a
-// batch must get the weights the whole batch would get).
+// batch must get the weights the whole batch would get); a batch at hand that is larger than `T_as` decides for itself,
+// because the logits buffer holds four parts of tc_split_rows() tokens at most.  The 148 SMs are a constant of the part,
+// not those of the device at hand: the rule must not differ between the ranks that route slices of one batch.
 constexpr int R_K_PARTS = 4;
 int tc_split_rows(int D, int E) { return D >= R_K_PARTS * 8 * R_BK ? 148 / R_K_PARTS / ceil_div(E, 64) * BM : 0; }   // batches up to this
-int tc_k_parts(int T_as, int D, int E) { return T_as <= tc_split_rows(D, E) ? R_K_PARTS : 1; }
+int tc_k_parts(int T, int T_as, int D, int E) { return std::max(T, T_as) <= tc_split_rows(D, E) ? R_K_PARTS : 1; }
 // (sized so that a batch never needs less scratch than a smaller one)
 TcScratch tc_layout(int T, int D, int E) {
   TcScratch s;
@@ -488,7 +490,7 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
                      cudaStream_t st) {
   BWMOE_REQUIRE(scratch != nullptr && aligned16(scratch), BWMOE_ERR_WORKSPACE, "router: scratch buffer required");
   BWMOE_REQUIRE(aligned16(x) && aligned16(wg), BWMOE_ERR_BAD_ALIGN, "router: pointers must be 16-byte aligned");
-  const int k_parts = tc_k_parts(T_as, D, E);
+  const int k_parts = tc_k_parts(T, T_as, D, E);
   const TcScratch L = tc_layout(T, D, E);
   uint8_t* base = static_cast<uint8_t*>(scratch);
   auto* wgt = reinterpret_cast<__nv_bfloat16*>(base + L.wgt);

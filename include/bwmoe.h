@@ -132,6 +132,7 @@ int bwmoe_router(const void* d_x, const void* d_w_gate, int T, int D, int E, int
  * rank routes its own tokens).  The routing kernels - chosen by batch size - select the same experts always,
  * but their fp32 weights can differ in the last bits; with T_as the slice is routed by the kernel the whole
  * batch would get, so that its weights equal, bit for bit, those of the whole batch routed in one call.
+ * T_as is at least T for that; a smaller one (0: T itself) is a valid choice of kernel and promises no such equality.
  * No counterpart in the reference (single GPU).
  */
 size_t bwmoe_router_scratch_bytes_as(int T, int D, int E, int K, int T_as);

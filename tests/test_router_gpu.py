@@ -140,3 +140,25 @@ def test_a_slice_routed_as_the_whole_batch_gets_the_whole_batch_weights():
             w_own, i_own = bw.top_k_router(x[s0:s0 + part].contiguous(), w, K)      # its own kernel: same experts
             assert torch.equal(i_own, i_all[s0:s0 + part])
             torch.testing.assert_close(w_own, w_all[s0:s0 + part], rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("T,D,E,K,T_as", [(4096, 2048, 256, 8, 128), (4096, 2048, 256, 8, 1024), (8192, 2048, 64, 6, 128),
+                                          (8192, 4096, 8, 2, 1024), (200, 2048, 64, 6, 128)])
+def test_a_batch_larger_than_as_batch_stays_inside_its_scratch(T, D, E, K, T_as):
+    """A batch may be routed as a smaller one.  The scratch is a part of a larger allocation whose rest has to stay as it
+    was (large enough for the logits of four K parts, so that too large a write shows here and nowhere else)."""
+    import blackwell_moe_b200 as bw
+    from blackwell_moe_b200 import _lib
+    lib = bw.lib()
+    g = torch.Generator().manual_seed(T + T_as)
+    x = torch.randn(T, D, generator=g).to(BF16).cuda()
+    w = (torch.randn(D, E, generator=g) * 0.02).to(BF16).cuda()
+    need = lib.bwmoe_router_scratch_bytes_as(T, D, E, K, T_as)
+    buf = torch.full((need + 4 * 4 * T * ((E + 15) // 16 * 16),), 0x5A, dtype=torch.uint8, device="cuda")
+    wt = torch.empty((T, K), device="cuda")
+    idx = torch.empty((T, K), dtype=torch.int32, device="cuda")
+    _lib.check(lib.bwmoe_router_as(x.data_ptr(), w.data_ptr(), T, D, E, K, T_as, wt.data_ptr(), idx.data_ptr(), None,
+                                   buf.data_ptr(), need, torch.cuda.current_stream().cuda_stream))
+    assert bool((buf[need:] == 0x5A).all())
+    wr, ir = bw.top_k_router(x, w, K)
+    assert torch.equal(idx, ir) and torch.equal(wt, wr)         # (both sizes get the tensor-core kernel)
