@@ -153,8 +153,9 @@ size_t router_tc_scratch_bytes(int T, int D, int E);
 int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
                      float* row_amax, int32_t* status, void* scratch, int T_as, void* zeroed_head,
                      cudaStream_t st);
-int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
-                           const int32_t* list, const int32_t* count, cudaStream_t st);
+int launch_router_fallback(const void* x, const void* wg, const void* wgt, int D, int E, int K, const RouteRows& out,
+                           const int32_t* list, const int32_t* count, const void* candidates, int ld_candidates,
+                           cudaStream_t st);
 size_t plan_scratch_bytes(int T, int E, int K);
 int launch_plan(const int32_t* indices, const float* row_amax, int T, int E, int K, int32_t* offsets,
                 int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax, int32_t* status,

@@ -586,18 +586,49 @@ router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 }
 
 // Exact (fp64) routing of the tokens in a device-side list; used behind the tensor-core router
-// for tokens whose candidate list overflowed.  Blocks stride over the list.
+// for tokens whose candidate list overflowed.  Blocks stride over the list.  An entry ~token has its candidates at
+// row `token` of `candidates` (their number, then their ids): the other experts cannot be among its K best, and a warp
+// per candidate along the transposed gate takes a tenth of the time of the whole gate matrix (35 us for a single token).
 __global__ void __launch_bounds__(256)
-router_fallback_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int D, int E,
-                       int K, const RouteRows out, const int32_t* __restrict__ list,
-                       const int32_t* __restrict__ count) {
+router_fallback_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg,
+                       const __nv_bfloat16* __restrict__ wgt, int D, int E, int K, const RouteRows out,
+                       const int32_t* __restrict__ list, const int32_t* __restrict__ count,
+                       const int32_t* __restrict__ candidates, int ld_candidates) {
   chain_wait();
   __shared__ float lg[256];
   __shared__ double dsum[256];
   const int n = *count;
   for (int f = blockIdx.x; f < n; f += gridDim.x) {
-    const int tok = list[f];
-    exact_logits_block(x + (size_t)tok * D, wg, D, E, lg, dsum);
+    const int entry = list[f], tok = entry < 0 ? ~entry : entry;
+    const __nv_bfloat16* xrow = x + (size_t)tok * D;
+    if (entry < 0) {
+      const int32_t* cand = candidates + (size_t)tok * ld_candidates;
+      const int n_cand = cand[0], lane = threadIdx.x & 31;
+      for (int e = threadIdx.x; e < E; e += blockDim.x) lg[e] = -INFINITY;
+      __syncthreads();
+      for (int c = threadIdx.x >> 5; c < n_cand; c += blockDim.x >> 5) {
+        const int e = cand[1 + c];
+        const __nv_bfloat16* wrow = wgt + (size_t)e * D;
+        double a = 0.0;
+#pragma unroll 2
+        for (int d = lane * 8; d < D; d += 256) {            // D is a multiple of 64 and the rows are 16-byte aligned here
+          const uint4 xr = *reinterpret_cast<const uint4*>(xrow + d), wr = *reinterpret_cast<const uint4*>(wrow + d);
+          const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&xr);
+          const __nv_bfloat162* pw = reinterpret_cast<const __nv_bfloat162*>(&wr);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 fx = __bfloat1622float2(px[j]), fw = __bfloat1622float2(pw[j]);
+            a = fma((double)fx.x, (double)fw.x, a);
+            a = fma((double)fx.y, (double)fw.y, a);
+          }
+        }
+        for (int off = 16; off; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        if (lane == 0) lg[e] = (float)a;
+      }
+      __syncthreads();
+    } else {
+      exact_logits_block(xrow, wg, D, E, lg, dsum);
+    }
     if (threadIdx.x < 32)
       select_token(lg, E, K, 0.f, -1.f, out, (size_t)tok, threadIdx.x);
     __syncthreads();
@@ -606,11 +637,12 @@ router_fallback_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
 
 }  // namespace
 
-int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
-                           const int32_t* list, const int32_t* count, cudaStream_t st) {
-  (void)T;
+int launch_router_fallback(const void* x, const void* wg, const void* wgt, int D, int E, int K, const RouteRows& out,
+                           const int32_t* list, const int32_t* count, const void* candidates, int ld_candidates,
+                           cudaStream_t st) {
   BWMOE_CUDA_OK(launch_chained(router_fallback_kernel, dim3(64), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x),
-                                             static_cast<const __nv_bfloat16*>(wg), D, E, K, out, list, count));
+                               static_cast<const __nv_bfloat16*>(wg), static_cast<const __nv_bfloat16*>(wgt), D, E, K, out, list,
+                               count, static_cast<const int32_t*>(candidates), ld_candidates));
   BWMOE_CUDA_OK(cudaGetLastError());
   return BWMOE_OK;
 }

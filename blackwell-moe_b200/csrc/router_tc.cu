@@ -17,7 +17,8 @@
 //                              compensated fp32 sum of the SIMT routers (error bound known), and in
 //                              fp64 if still within that bound of each other; the final top-K is
 //                              read off the mixed list.  A token for which an expert beyond the 12 best
-//                              may be a candidate is recomputed over all experts by the exact fallback kernel.
+//                              may be a candidate is recomputed over all experts by the exact fallback kernel,
+//                              and one that is in doubt only because of the longest column over its candidates.
 // An expert outside the candidate set has an exact logit below that of K candidates, so the
 // result equals the exact selection.
 #include "sm100_gemm.cuh"
@@ -239,7 +240,7 @@ __device__ __forceinline__ void kahan_add_r(float& sum, float& comp, float y) {
 template <int EJ>   // 32 * EJ >= E: logits each lane holds
 __global__ void __launch_bounds__(256)
 refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wgt,
-              const float* __restrict__ wnorm2, const float* __restrict__ logits, int ld_logits, int k_parts, int T, int D,
+              const float* __restrict__ wnorm2, float* logits, int ld_logits, int k_parts, int T, int D,
               int E, int K, const RouteRows out, float* __restrict__ row_amax,
               int32_t* __restrict__ fallback_count, int32_t* __restrict__ fallback_list) {
   chain_wait();
@@ -325,16 +326,30 @@ refine_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   for (int off = 16; off; off >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, off));
   const unsigned in_mask = __ballot_sync(0xffffffffu, lane < n_list && cv + t_mine >= low);
   bool settled = (in_mask & ((1u << K) - 1u)) == (1u << K) - 1u;      // (not so with NaN or infinite logits)
+  bool over = false;
   if (n_list == L_CAND && E > L_CAND && settled) {        // the list was cut off: could an expert outside it be a candidate?
     float rest = 0.f;                                     // the longest column among those
 #pragma unroll
     for (int j = 0; j < EJ; ++j)
       if (key[j] != 0u) rest = fmaxf(rest, wnorm2[lane + 32 * j]);
     for (int off = 16; off; off >>= 1) rest = fmaxf(rest, __shfl_xor_sync(0xffffffffu, rest, off));
-    settled = __shfl_sync(0xffffffffu, cv, L_CAND - 1) + kTcTrust * xnorm * sqrtf(rest) < low;
+    const float last = __shfl_sync(0xffffffffu, cv, L_CAND - 1);
+    settled = last + kTcTrust * xnorm * sqrtf(rest) < low;
+    over = last >= kth - t2;                              // it could by the bound of the largest norm
   }
   if (!settled) {
     if (lane == 0) fallback_list[atomicAdd(fallback_count, 1)] = tok;      // all-expert exact kernel
+    return;
+  }
+  if (over) {
+    // To the exact kernel as well - its logits, and so its weights, are better than the tensor cores' - but with the
+    // candidates only: their number and ids take the place of the token's logits.
+    int32_t* cand = reinterpret_cast<int32_t*>(logits + (size_t)tok * ld_logits);
+    if ((in_mask >> lane) & 1u) cand[1 + __popc(in_mask & ((1u << lane) - 1u))] = ci;
+    if (lane == 0) {
+      cand[0] = __popc(in_mask);
+      fallback_list[atomicAdd(fallback_count, 1)] = ~tok;
+    }
     return;
   }
   // ---- candidates whose error intervals overlap need exact logits.  Neighbours in the list tell whether there are any
@@ -481,10 +496,6 @@ bool router_tc_applicable(int T, int D, int E, int K) {
 
 size_t router_tc_scratch_bytes(int T, int D, int E) { return tc_layout(T, D, E).total; }
 
-// Exact router for the tokens the candidate list could not settle (device list, count read on the device).
-int launch_router_fallback(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
-                           const int32_t* list, const int32_t* count, cudaStream_t st);
-
 int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, const RouteRows& out,
                      float* row_amax, int32_t* status, void* scratch, int T_as, void* zeroed_head,
                      cudaStream_t st) {
@@ -535,7 +546,7 @@ int launch_router_tc(const void* x, const void* wg, int T, int D, int E, int K, 
     BWMOE_CUDA_OK(launch_chained(refine_kernel<8>, dim3(rgrid), dim3(256), 0, st, xb, wgt, wnorm2, logits, p.n_mma, k_parts, T, D, E, K, out, row_amax,
                                             fb_count, fb_list));
   BWMOE_CUDA_OK(cudaGetLastError());
-  return launch_router_fallback(x, wg, T, D, E, K, out, fb_list, fb_count, st);
+  return launch_router_fallback(x, wg, wgt, D, E, K, out, fb_list, fb_count, logits, p.n_mma, st);
 }
 
 }  // namespace bwmoe

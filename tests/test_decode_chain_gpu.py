@@ -142,6 +142,26 @@ def test_router_with_columns_of_very_different_length(T, D, E, K):
     torch.testing.assert_close(wt.cpu(), wr, rtol=1e-3, atol=1e-4)
 
 
+@pytest.mark.parametrize("T,D,E,K", [(2000, 1024, 128, 8), (300, 2048, 256, 8), (1100, 512, 64, 3), (1030, 256, 16, 4)])
+def test_tokens_that_one_long_column_puts_in_doubt_get_exact_weights(T, D, E, K):
+    """One column is so long that, trusted to its norm, more experts than the candidate list holds might reach the K best.
+    Such tokens carry the weights of the fp64 kernels bit for bit, whether their own experts' norms settle them or not."""
+    import blackwell_moe_b200 as bw
+    g = torch.Generator().manual_seed(D)
+    x = torch.randn(T, D, generator=g).to(BF16)
+    w = (torch.randn(D, E, generator=g) * 0.02).to(BF16)
+    x[:, 0], w[0, E // 3] = 0.0, 250.0                   # (the feature is off: the expert's logit stays ordinary)
+    wt, idx = bw.top_k_router(x.cuda(), w.cuda(), K)
+    we, ie = bw.top_k_router(x.cuda(), w.cuda(), K, as_batch=32)             # the decode kernel: fp64 sums
+    assert torch.equal(idx, ie)
+    logits = x.double() @ w.double()
+    trust = 2.0 ** -13 * x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=0).max()
+    near = (logits >= logits.topk(K, dim=1).values[:, -1:] - 0.95 * trust).sum(1)
+    doubt = near > 12
+    assert int(doubt.sum()) > T // 4
+    assert torch.equal(wt.cpu()[doubt], we.cpu()[doubt])
+
+
 @pytest.mark.parametrize("T,D,K", [(1, 8, 1), (5, 264, 2), (3, 256, 5), (7, 1032, 8), (4, 512, 32), (3, 72, 33), (2, 128, 70)])
 def test_combine_stage_with_ragged_rows_and_any_number_of_slots(T, D, K):
     """The combine entry point: row widths that leave lanes idle, up to 2, 4 and 8 rows in flight, more slots than a warp
