@@ -722,18 +722,23 @@ down_combine_from_partials_kernel(const float* __restrict__ partial, int S, int 
 }
 
 // Split-K is for small batches, where a few experts x column blocks cannot occupy every SM (fewer than four rounds of
-// tiles).  The K loop of each tile is cut into the number of pieces that makes the longest CTA shortest - rounds of pieces
-// x K blocks of a piece - with one per cent per piece for the slabs: two experts of the Mixtral shape (224 gate/up tiles of
-// 32 blocks) take 13 rounds of 4 blocks instead of 5 of 11 (56 -> 53 us), eight of the DeepSeek shape 5 of 2 instead of 4 of 3.
+// tiles).  The K loop of each tile is cut into at least as many pieces as make four rounds, and beyond that into the number
+// that makes the longest CTA shortest - rounds of pieces x K blocks of a piece - with one per cent per piece for the slabs:
+// two experts of the Mixtral shape (224 gate/up tiles of 32 blocks) take 13 rounds of 4 blocks instead of 5 of 11 (56 -> 53
+// us), eight of the DeepSeek shape 5 of 2 instead of 4 of 3.  Never fewer pieces than four rounds need: the tensor core
+// truncates at every step, so a sum's error grows with the length of its piece (four rows of K = 14336 in pieces of 56
+// blocks instead of 14: 8.0e-4 of the results not the correctly rounded ones, 2.2e-4 before).
 struct SplitPlan {
   int split_k, k_per_split;
 };
 SplitPlan choose_split(int M, int E, int k_blocks, int n_tiles) {
   SplitPlan sp{1, k_blocks};
   const long long tiles = (long long)std::min(M, E) * n_tiles;      // one row tile per active expert, at most
-  if (M > kSplitMaxRows || tiles >= 4ll * sm_count()) return sp;
+  const long long full = 4ll * sm_count();
+  if (M > kSplitMaxRows || tiles >= full) return sp;
+  const int most = std::min(kSplitMax, k_blocks / 2);
   double best = 0.0;
-  for (int n = 2; n <= std::min(kSplitMax, k_blocks / 2); ++n) {
+  for (int n = (int)std::min<long long>(most, (full + tiles - 1) / tiles); n >= 2 && n <= most; ++n) {
     const int per = ceil_div(k_blocks, n), pieces = ceil_div(k_blocks, per);
     const long long rounds = (tiles * pieces + sm_count() - 1) / sm_count();
     const double cost = (double)(rounds * per) * (1.0 + 0.01 * pieces);

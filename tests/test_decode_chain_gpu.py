@@ -162,6 +162,38 @@ def test_tokens_that_one_long_column_puts_in_doubt_get_exact_weights(T, D, E, K)
     assert torch.equal(wt.cpu()[doubt], we.cpu()[doubt])
 
 
+@pytest.mark.parametrize("M,E,D,H", [(4, 4, 4096, 3584), (2, 2, 4096, 7168), (8, 8, 2048, 1408), (1, 1, 1024, 2048), (3, 5, 272, 640)])
+def test_split_k_pieces_are_no_longer_than_four_rounds_of_tiles_make_them(M, E, D, H):
+    """A piece is one fp32 sum of the tensor core, which truncates at every step: the longer, the less exact.  The slabs of
+    the partial sums - one per piece, in scratch that starts at zero - are counted, and their sum is compared with fp64."""
+    from blackwell_moe_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(M + H)
+    hq = torch.randn(M, H, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    w = torch.randn(E, H, D, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    offsets = torch.tensor([min(e, M) for e in range(E)] + [M], dtype=torch.int32, device="cuda")
+    one, status = torch.ones(E, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    y = torch.empty(M, D, dtype=BF16, device="cuda")
+    scratch = torch.zeros(lib.bwmoe_gemm_scratch_bytes(M, D, H, E), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.bwmoe_down(hq.data_ptr(), offsets.data_ptr(), one.data_ptr(), w.data_ptr(), one.data_ptr(), M, D, H, E,
+                              y.data_ptr(), status.data_ptr(), scratch.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    slabs = scratch[:8 * M * D * 4].view(torch.float32).view(8, M, D)
+    pieces = int((slabs != 0).flatten(1).any(1).sum())
+    k_blocks, tiles = -(-H // 128), min(M, E) * -(-D // 256)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    least = min(8, k_blocks // 2, -(-4 * sms // tiles))
+    assert pieces >= -(-k_blocks // -(-k_blocks // least))
+    assert int(status[0]) == 0
+    expert = [max(e for e in range(E) if offsets[e] <= m < offsets[e + 1]) for m in range(M)]
+    want = torch.stack([hq[m].double() @ w[e].double() for m, e in enumerate(expert)])
+    # 4 steps per K block, each off by at most 2^-23 of a partial sum of deviation sqrt(H) or less, hardly above five times that
+    assert float((slabs.double().sum(0) - want).abs().max()) < 4 * k_blocks * 2.0 ** -23 * 5 * H ** 0.5
+    total = torch.zeros(M, D, device="cuda")
+    for slab in slabs:
+        total += slab
+    assert torch.equal(y, total.to(BF16))
+
+
 @pytest.mark.parametrize("T,D,K", [(1, 8, 1), (5, 264, 2), (3, 256, 5), (7, 1032, 8), (4, 512, 32), (3, 72, 33), (2, 128, 70)])
 def test_combine_stage_with_ragged_rows_and_any_number_of_slots(T, D, K):
     """The combine entry point: row widths that leave lanes idle, up to 2, 4 and 8 rows in flight, more slots than a warp
