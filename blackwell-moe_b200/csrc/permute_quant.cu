@@ -574,6 +574,35 @@ combine_peers_kernel(const PeerPtrs src, const int32_t* __restrict__ pos, const 
   reinterpret_cast<uint4*>(out + (size_t)t * D)[v] = o;
 }
 
+// Glue and rounding of one vector of a token's result, from the fp32 sums over its routed and its always-on rows.
+__device__ __forceinline__ void store_combined(float (&acc)[8], const float (&tail)[8], int t, int v, int D,
+                                               __nv_bfloat16* __restrict__ out, float scale,
+                                               const __nv_bfloat16* __restrict__ residual, int n_tail) {
+  if (scale != 1.0f) {     // bf16 tensor times a Python scalar: torch multiplies in fp32 by the unrounded scalar
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = bf16_round(bf16_round(acc[i]) * scale);
+  }
+  if (residual != nullptr) {
+    const uint4 raw = reinterpret_cast<const uint4*>(residual + (size_t)t * D)[v];
+    const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(q[i]);
+      acc[2 * i] = bf16_round(acc[2 * i]) + f.x;
+      acc[2 * i + 1] = bf16_round(acc[2 * i + 1]) + f.y;
+    }
+  }
+  if (n_tail > 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = bf16_round(acc[i]) + bf16_round(tail[i]);
+  }
+  uint4 o;
+  __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+  reinterpret_cast<uint4*>(out + (size_t)t * D)[v] = o;
+}
+
 // ---- out[t,:] = bf16( sum_k float( bf16( y[pos[t*K+k],:] * bf16(w[t,k]) ) ) ) ----
 // Optional tail (the block glue of FP8MoELayer.forward, src/blackwell_moe/runtime/deepseek_patch.py:51-53):
 //   out = bf16( bf16(routed * scale) + residual ) with routed = the bf16 sum above.
@@ -632,30 +661,53 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ 
       }
     }
   }
-  if (!v_ok) return;
-  if (scale != 1.0f) {     // bf16 tensor times a Python scalar: torch multiplies in fp32 by the unrounded scalar
+  if (v_ok) store_combined(acc, tail, t, v, D, out, scale, residual, n_tail);
+}
+
+// The same for rows that are short or fill warps badly: one thread per vector of a token's row, no lane idle, three rows
+// at a time (their vectors are all requested before the first is used).
+template <bool PREWEIGHTED>
+__global__ void __launch_bounds__(256)
+combine_flat_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ pos,
+                    const float* __restrict__ weights, int T, int D, int K, __nv_bfloat16* __restrict__ out,
+                    float scale, const __nv_bfloat16* __restrict__ residual, int n_tail) {
+  chain_wait();
+  const int vec_per_row = D / 8;
+  const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= (size_t)T * vec_per_row) return;
+  const int t = (int)(gid / vec_per_row), v = (int)(gid % vec_per_row);
+  float acc[8], tail[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = bf16_round(bf16_round(acc[i]) * scale);
-  }
-  if (residual != nullptr) {
-    const uint4 raw = reinterpret_cast<const uint4*>(residual + (size_t)t * D)[v];
-    const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f, tail[i] = 0.f;
+  constexpr int kRows = 3;
+  for (int k0 = 0; k0 < K; k0 += kRows) {
+    int p[kRows];
+    float w[kRows];
+    uint4 raw[kRows];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __bfloat1622float2(q[i]);
-      acc[2 * i] = bf16_round(acc[2 * i]) + f.x;
-      acc[2 * i + 1] = bf16_round(acc[2 * i + 1]) + f.y;
+    for (int j = 0; j < kRows; ++j) {
+      const size_t at = (size_t)t * K + k0 + j;
+      p[j] = k0 + j < K ? pos[at] : -1;
+      w[j] = k0 + j < K && !PREWEIGHTED ? weights[at] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+      raw[j] = p[j] >= 0 ? reinterpret_cast<const uint4*>(y + (size_t)p[j] * D)[v] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      if (p[j] < 0) continue;
+      const float wk = bf16_round(w[j]);
+      const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float2 f = __bfloat1622float2(q[i]);
+        if (!PREWEIGHTED) f = __bfloat1622float2(__floats2bfloat162_rn(f.x * wk, f.y * wk));
+        if (k0 + j < K - n_tail) acc[2 * i] += f.x, acc[2 * i + 1] += f.y;
+        else                     tail[2 * i] += f.x, tail[2 * i + 1] += f.y;
+      }
     }
   }
-  if (n_tail > 0) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = bf16_round(acc[i]) + bf16_round(tail[i]);
-  }
-  uint4 o;
-  __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
-  reinterpret_cast<uint4*>(out + (size_t)t * D)[v] = o;
+  store_combined(acc, tail, t, v, D, out, scale, residual, n_tail);
 }
 
 // What the pipeline needs of a batch whose routing the caller did: max|x| of every row, the routing copied into the
@@ -906,12 +958,22 @@ int launch_combine(const void* y, const int32_t* pos, const float* weights, int 
   BWMOE_REQUIRE(T > 0 && D > 0 && K > 0 && D % 8 == 0, BWMOE_ERR_BAD_SHAPE, "combine: T=%d D=%d K=%d", T, D, K);
   BWMOE_REQUIRE(y && pos && weights && out, BWMOE_ERR_NULL, "combine: null pointer");
   BWMOE_REQUIRE(aligned16(y) && aligned16(out), BWMOE_ERR_BAD_ALIGN, "combine: pointers must be 16-byte aligned");
-  const size_t warps = (size_t)T * ceil_div(D / 8, 32);
-  const dim3 grid((unsigned)((warps + 7) / 8)), block(256);
+  // A thread per vector where warps of one token would be a quarter empty or more: rows of up to 192 columns and a few
+  // sizes above (20000 tokens, K = 8: 64 columns 7.1 us against 16.5, 192 15.1 and 18.2, 384 35.5 and 34.3; K = 6, 576 40.5 and
+  // 44.2; where they are full, 256 columns 22.2 and 19.1, 1024 86.5 and 67.9).
+  const int vecs = D / 8, warps_per_row = ceil_div(vecs, 32);
+  const bool flat = 4 * vecs <= 3 * 32 * warps_per_row;
+  const size_t threads = (size_t)T * (flat ? vecs : 32 * warps_per_row);
+  const dim3 grid((unsigned)((threads + 255) / 256)), block(256);
   auto launch = [&](auto kernel) {
     return launch_chained(kernel, grid, block, 0, st, static_cast<const __nv_bfloat16*>(y), pos, weights, T, D, K,
                           static_cast<__nv_bfloat16*>(out), scale, static_cast<const __nv_bfloat16*>(residual), n_tail);
   };
+  if (flat) {
+    BWMOE_CUDA_OK(preweighted ? launch(combine_flat_kernel<true>) : launch(combine_flat_kernel<false>));
+    BWMOE_CUDA_OK(cudaGetLastError());
+    return BWMOE_OK;
+  }
   // as many rows in flight as a token has, eight at most (their registers then cost occupancy)
   if (preweighted) BWMOE_CUDA_OK(K <= 2 ? launch(combine_kernel<true, 2>) : K <= 4 ? launch(combine_kernel<true, 4>) : launch(combine_kernel<true, 8>));
   else             BWMOE_CUDA_OK(K <= 2 ? launch(combine_kernel<false, 2>) : K <= 4 ? launch(combine_kernel<false, 4>) : launch(combine_kernel<false, 8>));

@@ -51,10 +51,11 @@ def test_block_forward_at_the_edges_of_the_dispatch(T, D, E, K, H):
     assert torch.equal(call(), out)                     # sums in a fixed order
 
 
-@pytest.mark.parametrize("T", [1, 8, 9, 150])           # 8, 64, 72 and 1200 rows: fused and separate requantisation
-def test_always_on_experts_share_one_scale_and_follow_the_routed_slots(T):
+# 8, 64, 72 and 1200 rows: fused and separate requantisation; both forms of the combine (rows of 512 and 272 columns)
+@pytest.mark.parametrize("T,D", [(1, 512), (8, 512), (9, 512), (150, 512), (9, 272), (150, 272)])
+def test_always_on_experts_share_one_scale_and_follow_the_routed_slots(T, D):
     import blackwell_moe_b200 as bw
-    D, E, K, H, S = 512, 16, 6, 256, 2
+    E, K, H, S = 16, 6, 256, 2
     inp = make_inputs(T, D, E, K, H, seed=T + 3)
     shared = [oracle.quant_fp8_e4m3((torch.randn(a, b, generator=torch.Generator().manual_seed(i)) * 0.02).to(BF16))
               for i, (a, b) in enumerate(((D, S * H), (D, S * H), (S * H, D)))]
@@ -196,8 +197,8 @@ def test_split_k_pieces_are_no_longer_than_four_rounds_of_tiles_make_them(M, E, 
 
 @pytest.mark.parametrize("T,D,K", [(1, 8, 1), (5, 264, 2), (3, 256, 5), (7, 1032, 8), (4, 512, 32), (3, 72, 33), (2, 128, 70)])
 def test_combine_stage_with_ragged_rows_and_any_number_of_slots(T, D, K):
-    """The combine entry point: row widths that leave lanes idle, up to 2, 4 and 8 rows in flight, more slots than a warp
-    has lanes, slots without a row - the fixed-order fp32 sum of bf16 products, bit for bit."""
+    """The combine entry point: row widths that leave lanes idle (both forms of the kernel), up to 2, 4 and 8 rows in flight,
+    more slots than a warp has lanes, slots without a row - the fixed-order fp32 sum of bf16 products, bit for bit."""
     from blackwell_moe_b200 import _lib
     lib = _lib.lib()
     g = torch.Generator().manual_seed(T * K)
