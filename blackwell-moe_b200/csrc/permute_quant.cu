@@ -155,7 +155,7 @@ plan_rank_kernel(const int32_t* __restrict__ indices, int M, int E, int per_bloc
   }
 }
 
-// ---- all three passes in one block, for at most 1024 slots (decode-sized batches) ----
+// ---- both passes in one block, for at most 1024 slots (decode-sized batches) ----
 struct SmallPlan {
   int start[kMaxE + 1];        // first row of each expert; [E] = rows that exist
   unsigned int amax[kMaxE];    // bits of the segment's max|x|
@@ -384,11 +384,13 @@ scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restr
 // The plan of a decode-sized batch (at most 1024 slots) and the quantisation of its rows in one launch.  Every block
 // works the plan out for itself - the batch's routing is a few KiB and the scans take about a microsecond, less than a
 // kernel boundary - block 0 publishes it, and each block then quantises its tokens into their K rows, one thread per
-// (slot of the token, 16 elements).  A token's first pieces are requested before the plan starts.
+// (slot of one of the tokens, 16 elements).  The block's first pieces are requested before the plan starts.  (One token
+// after the other instead of all their slots in a row: 54.8 us for a call of 1024 tokens x 1 slot of 1024, 64 threads of
+// 1024 at work at a time.)
 // GROUPS: the block-scale recipe - one scale per 128 elements, independent of the expert (eight neighbouring threads
 // share the maximum), inverse scales to x_inv; otherwise the scale of the row's segment.
 template <bool GROUPS>
-__global__ void __launch_bounds__(kPlanThreads)
+__global__ void __launch_bounds__(kPlanThreads, 1)
 plan_quant_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ indices,
                   const float* __restrict__ row_amax, const float* __restrict__ weights, int T, int D, int E, int K,
                   int32_t* __restrict__ offsets, int32_t* __restrict__ pos, int32_t* __restrict__ row_slot,
@@ -400,17 +402,27 @@ plan_quant_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict
   __shared__ int s_row[kPlanThreads];
   __shared__ float s_scale[kPlanThreads];          // the scale of each slot's segment
   const int pieces = D / 16, groups = (D + 127) / 128, padded = groups * 8;     // threads of one slot: whole groups
-  const int items = K * padded;
+  const int tokens = (T - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;      // this block's: blockIdx.x, + gridDim.x, ...
+  const int items = tokens * K * padded;
+  // item -> its token, its slot of the batch and its piece (`pieces`: none)
+  auto locate = [&](int item, int& t, int& slot, int& c) {
+    const int n = item / padded, j = tokens == 1 ? 0 : n / K;
+    t = (int)blockIdx.x + j * (int)gridDim.x;
+    slot = item < items ? t * K + n - j * K : 0;
+    c = item < items ? item - n * padded : pieces;
+  };
   // x was complete before the kernel in front of this one ran (it is an input of that kernel as well)
   auto load_piece = [&](int t, int c, uint4& r0, uint4& r1) {
     r0 = r1 = make_uint4(0u, 0u, 0u, 0u);
-    if (t < T && c < pieces) {
+    if (c < pieces) {
       const uint4* in = reinterpret_cast<const uint4*>(x + (size_t)t * D) + 2 * c;
       r0 = in[0], r1 = in[1];
     }
   };
-  uint4 p0, p1;
-  load_piece(blockIdx.x, (int)threadIdx.x < items ? (int)threadIdx.x % padded : pieces, p0, p1);
+  int t, slot, c;
+  uint4 r0, r1;
+  locate((int)threadIdx.x, t, slot, c);
+  load_piece(t, c, r0, r1);
   chain_wait();
   const int M = T * K;
   {
@@ -424,42 +436,40 @@ plan_quant_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict
     }
   }
   __syncthreads();
-  for (int t = blockIdx.x; t < T; t += gridDim.x) {
-    for (int base = 0; base < items; base += kPlanThreads) {       // uniform for the block: the shuffles below need it
-      const int item = base + threadIdx.x;
-      const int k = item < items ? item / padded : 0, c = item < items ? item - k * padded : pieces;
-      uint4 r0 = p0, r1 = p1;
-      if (t != (int)blockIdx.x || base > 0) load_piece(t, c, r0, r1);
-      const int row = s_row[t * K + k];
-      float scale, inv = 0.f;
-      if constexpr (GROUPS) {
-        const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-        float m = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
-        for (int off = 4; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off, 8));
-        m = fmaxf(m, kGroupAmaxFloor);
-        scale = __fmul_rn(__frcp_rn(m), kFp8Max);
-        inv = __fdiv_rn(m, kFp8Max);
-      } else {
-        scale = s_scale[t * K + k];
-      }
-      if (c < pieces && row >= 0) {                  // row < 0: slot with an out-of-range expert
-        uint4 codes;
-        if constexpr (GROUPS) {                      // min/max clamp as in quant_group_rows_kernel (it decides what NaN becomes)
-          codes = make_uint4(e4m3x4_clamped(r0.x, r0.y, scale), e4m3x4_clamped(r0.z, r0.w, scale),
-                             e4m3x4_clamped(r1.x, r1.y, scale), e4m3x4_clamped(r1.z, r1.w, scale));
-          if ((c & 7) == 0) x_inv[(size_t)row * groups + (c >> 3)] = inv;
-        } else {
-          const unsigned long long s2 = splat2(scale);
-          codes = make_uint4(e4m3x4_scaled(r0.x, r0.y, s2), e4m3x4_scaled(r0.z, r0.w, s2), e4m3x4_scaled(r1.x, r1.y, s2),
-                             e4m3x4_scaled(r1.z, r1.w, s2));
-        }
-        reinterpret_cast<uint4*>(dst + (size_t)row * D)[c] = codes;
-      }
-      __syncwarp();
+  for (int base = 0; base < items; base += kPlanThreads) {         // uniform for the block: the shuffles below need it
+    if (base > 0) {
+      locate(base + (int)threadIdx.x, t, slot, c);
+      load_piece(t, c, r0, r1);
     }
+    const int row = s_row[slot];
+    float scale, inv = 0.f;
+    if constexpr (GROUPS) {
+      const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
+      for (int off = 4; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off, 8));
+      m = fmaxf(m, kGroupAmaxFloor);
+      scale = __fmul_rn(__frcp_rn(m), kFp8Max);
+      inv = __fdiv_rn(m, kFp8Max);
+    } else {
+      scale = s_scale[slot];
+    }
+    if (c < pieces && row >= 0) {                    // row < 0: slot with an out-of-range expert
+      uint4 codes;
+      if constexpr (GROUPS) {                        // min/max clamp as in quant_group_rows_kernel (it decides what NaN becomes)
+        codes = make_uint4(e4m3x4_clamped(r0.x, r0.y, scale), e4m3x4_clamped(r0.z, r0.w, scale),
+                           e4m3x4_clamped(r1.x, r1.y, scale), e4m3x4_clamped(r1.z, r1.w, scale));
+        if ((c & 7) == 0) x_inv[(size_t)row * groups + (c >> 3)] = inv;
+      } else {
+        const unsigned long long s2 = splat2(scale);
+        codes = make_uint4(e4m3x4_scaled(r0.x, r0.y, s2), e4m3x4_scaled(r0.z, r0.w, s2), e4m3x4_scaled(r1.x, r1.y, s2),
+                           e4m3x4_scaled(r1.z, r1.w, s2));
+      }
+      reinterpret_cast<uint4*>(dst + (size_t)row * D)[c] = codes;
+    }
+    __syncwarp();
   }
 }
 
@@ -777,7 +787,7 @@ int launch_plan_quant(const void* x, const int32_t* indices, const float* row_am
                       int K, int32_t* offsets, int32_t* pos, int32_t* row_slot, int32_t* row_expert, float* seg_amax,
                       float* scales, int32_t* status, void* xq, float* row_w, float* x_inv, cudaStream_t st) {
   BWMOE_REQUIRE(plan_quant_applicable(T, E, K) && D % 16 == 0, BWMOE_ERR_BAD_SHAPE, "plan_quant: T=%d D=%d E=%d K=%d", T, D, E, K);
-  const dim3 grid((unsigned)std::min(T, 2 * sm_count())), block(kPlanThreads);     // two blocks of 1024 threads per SM
+  const dim3 grid((unsigned)std::min(T, sm_count())), block(kPlanThreads);     // (its registers allow no second block per SM)
   const size_t smem = small_plan_smem(E);
   auto xb = static_cast<const __nv_bfloat16*>(x);
   auto q = static_cast<uint8_t*>(xq);
