@@ -1,7 +1,7 @@
 """The kernels and dispatch rules of decode-sized calls at the sizes where they can go wrong, against the oracle: the plan
 and quantisation in one launch (up to 1024 slots) and the two-pass plan beyond, split-K post passes (up to 64 rows), the
-block-scale tiles that read back 8, 16 or 32 token columns and share their K blocks among the CTAs of a cluster (up to 8
-rows), always-on experts written by the router, caller-routed batches, and the router's candidate bounds."""
+block-scale tiles that read back 8, 16 or 32 token columns, always-on experts written by the router, caller-routed batches,
+and the router's candidate bounds."""
 
 import pytest
 import torch
@@ -24,8 +24,8 @@ def test_per_tensor_forward_at_the_edges_of_the_dispatch(T, D, E, K, H):
     check_against_oracle(inp, out, views, ref, inter)
 
 
-# one token: clusters of 4 (8 tiles of 8 K blocks), of 2 (40 and 64 tiles; 5 K blocks in unequal shares), none (down: 2 K
-# blocks); 8 rows in one expert; 9 rows: no clusters; segments of up to 8, 16 and 32 rows and beyond one 32-row tile
+# the kernel for up to 8 rows per expert on average: one token over few and many tiles, an odd number of K blocks, a single
+# expert, ragged D and H, several row tiles per expert; 1024 and 1025 slots
 @pytest.mark.parametrize("T,D,E,K,H", [(1, 1024, 16, 8, 128), (1, 1024, 16, 8, 640), (1, 2048, 128, 8, 768), (1, 640, 8, 3, 384),
                                        (2, 512, 8, 4, 256), (8, 512, 1, 1, 256), (9, 1024, 2, 1, 256), (24, 384, 8, 2, 576),
                                        (40, 512, 16, 3, 208), (70, 256, 32, 2, 144), (1024, 128, 256, 1, 128), (1025, 272, 160, 1, 128)])
@@ -49,6 +49,46 @@ def test_block_forward_at_the_edges_of_the_dispatch(T, D, E, K, H):
     assert oracle.rel_l1(v["y"], inter["y_perm"]) < 1e-2
     assert oracle.rel_l1(out.cpu(), ref) < 1e-2
     assert torch.equal(call(), out)                     # sums in a fixed order
+
+
+def _rows_per_expert(counts):
+    """Caller-routed batch of one slot per token in which expert e gets counts[e] rows, in no order."""
+    g = torch.Generator().manual_seed(sum(counts))
+    ids = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    ids = ids[torch.randperm(len(ids), generator=g)].to(torch.int32)[:, None]
+    return torch.rand(len(ids), 1, generator=g) + 0.5, ids
+
+
+# rows of the first expert: both sides of the 8, 16 and 32 columns that a tile reads back and holds, and of two tiles
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("D,H", [(512, 256), (400, 208)])
+def test_block_tiles_at_the_edges_of_what_they_read_back(rows, D, H):
+    _check_block_routed([rows, 0, 3] + [0] * 13, D, H)
+
+
+# 8 rows per expert on average are the last for the small kernel: 64 and 65 rows of 8 experts
+@pytest.mark.parametrize("counts", [[8] * 8, [8] * 7 + [9], [40, 0, 3, 9, 1, 11, 0, 0], [40, 0, 3, 9, 1, 11, 1, 0]])
+def test_block_kernels_on_both_sides_of_eight_rows_per_expert(counts):
+    _check_block_routed(counts, 384, 272)
+
+
+def _check_block_routed(counts, D, H):
+    import blackwell_moe_b200 as bw
+    wt, ids = _rows_per_expert(counts)
+    T, E = len(ids), len(counts)
+    inp = make_block_inputs(T, D, E, 1, H, seed=T + D)
+    c = to_cuda(inp)
+    out = bw.fp8_moe_forward_routed(c["x"], wt.cuda(), ids.cuda(), c["q_gate"], c["q_up"], c["q_down"],
+                                    c["inv_gate"], c["inv_up"], c["inv_down"])
+    v = {k: t.cpu() for k, t in bw.moe_stage_views("cuda:0", T, D, H, E, 1, block=True).items()}
+    inter = {}
+    ref = oracle.moe_forward_block_recipe(inp["x"], None, inp["q_gate"], inp["q_up"], inp["q_down"], inp["inv_gate"],
+                                          inp["inv_up"], inp["inv_down"], routing=(wt, ids), intermediates=inter)
+    assert int(v["status"][0]) == 0
+    assert torch.equal(v["offsets"], inter["offsets"]) and torch.equal(v["x_inv"], inter["x_inv"])
+    assert (v["hq"].view(torch.uint8) != inter["hq"].view(torch.uint8)).float().mean().item() < 0.02
+    assert max(oracle.rel_l1(v["y"][i], inter["y_perm"][i]) for i in range(T)) < 2e-2
+    assert oracle.rel_l1(out.cpu(), ref) < 1e-2
 
 
 # 8, 64, 72 and 1200 rows: fused and separate requantisation; both forms of the combine (rows of 512 and 272 columns)
@@ -222,23 +262,28 @@ def test_combine_stage_with_ragged_rows_and_any_number_of_slots(T, D, K):
 @pytest.mark.parametrize("T,E,block", [(1, 16, False), (40, 16, False), (1, 16, True), (100, 64, True), (600, 64, False)])
 def test_calls_can_be_captured_and_replayed(T, E, block):
     """The launch chain (cluster launches, programmatic edges, a memset only where the tensor-core router runs) in a CUDA
-    graph: a replay on new activations equals the plain call."""
+    graph, behind the kernel that makes the activations: a replay on new values equals the plain call on them."""
     import blackwell_moe_b200 as bw
     D, K, H = 512, 4, 256
     inp = make_block_inputs(T, D, E, K, H, seed=T) if block else make_inputs(T, D, E, K, H, seed=T)
     c = to_cuda(inp)
     s = "inv_" if block else "s_"
     w = (c["w_gate"], c["q_gate"], c["q_up"], c["q_down"], c[s + "gate"], c[s + "up"], c[s + "down"])
-    x = c["x"].clone()
+    source = c["x"].clone()
     stream = torch.cuda.Stream()
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
-        bw.fp8_moe_forward(x, *w, top_k=K)
+        bw.fp8_moe_forward(source * 2, *w, top_k=K)
         stream.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=stream):
-            out = bw.fp8_moe_forward(x, *w, top_k=K)
-    x.copy_(c["x"].flip(0))
+            out = bw.fp8_moe_forward(source * 2, *w, top_k=K)
     graph.replay()
     torch.cuda.synchronize()
-    assert torch.equal(out, bw.fp8_moe_forward(c["x"].flip(0).contiguous(), *w, top_k=K))
+    first = out.clone()
+    for seed in (1001, 1002):
+        source.copy_(torch.randn(T, D, generator=torch.Generator().manual_seed(seed)).to(BF16))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, bw.fp8_moe_forward(source * 2, *w, top_k=K))
+        assert not torch.equal(out, first)

@@ -1,4 +1,6 @@
-"""Scratch sizes never shrink as a batch grows: a buffer sized for the largest batch serves every smaller one."""
+"""Scratch of the plan and of the router never shrinks as a batch grows: a buffer sized for the largest batch serves every
+smaller one.  (The scratch of the split-K GEMMs, and with it a forward's workspace, is largest at 64 rows: it is sized per
+batch, or for the largest of the batches it serves.)"""
 
 import pytest
 

@@ -3,7 +3,7 @@
 Some callers cannot give the library a scratch buffer because they cannot
 allocate device memory where they call from (an allocator callback, a plugin
 that only receives its inputs and outputs, a loop that has frozen its memory
-pool).  For them the library carries a fixed 64 KiB scratch array of its own.
+pool).  For them the library carries a fixed 128 KiB scratch array of its own.
 This test drives that entry point through the C ABI and requires exactly the
 results of the regular entry point, three times in a row with different expert
 counts and block counts, every call large enough to take the multi-pass plan
