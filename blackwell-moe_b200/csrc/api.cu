@@ -93,7 +93,8 @@ namespace {
 constexpr size_t kAlign = 1024;
 inline size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
-// Workspace layout.  The first block (status .. amax_h) is cleared by one memset per call.
+// Workspace layout.  The first block (status .. router_head) has to be zero when the plan starts: the kernel in front of it
+// clears it where it has the time (router_token_kernel, routed_prepare_kernel), a memset where another router runs.
 struct Layout {
   size_t status, amax_x, amax_h, arrivals, router_head, zero_end;
   size_t offsets, scale_x, scale_h, topk_idx, topk_w, row_amax, pos, row_slot, row_expert, row_w;

@@ -33,15 +33,17 @@ inline cudaStream_t counted(cudaStream_t st) {
 
 // Programmatic dependent launch: a kernel launched through launch_chained() may be scheduled while the kernel
 // before it in the stream is still draining (its launch latency and block start-up overlap that tail).
-// Such a kernel executes chain_wait() before it touches global memory: the instruction returns when every
-// kernel it depends on has completed and its writes are visible.  A kernel that calls chain_wait() may
-// also be launched the ordinary way (the instruction then returns at once), but a kernel launched through
-// launch_chained() MUST call it.
+// chain_wait() returns when the kernel in front has completed and its writes are visible.  All threads of a chained
+// kernel call it: a kernel that ends without it could end before the one in front, and the kernel behind it would then
+// start too early.  A kernel that calls it may also be launched the ordinary way (the instruction returns at once).
+// Before the wait a kernel may touch only what the kernel in front neither writes nor, where it is written here, reads
+// (two do: plan_quant_kernel requests x, transpose_gate_kernel does all of its work).  That is sound because everything
+// BEFORE the kernel in front is complete by then, which in turn rests on every kernel of the chain waiting before it
+// lets the next one be scheduled - by ending, or by chain_next().
 //
 // chain_next(), called AFTER chain_wait(), lets the next kernel of the chain be scheduled as soon as every block of
 // this one has got that far: its blocks take the places that are free (or become free) and do what needs no
-// result of this kernel while this kernel still runs.  Since every kernel signals only behind its own wait, a
-// kernel that has been scheduled knows that everything BEFORE its direct predecessor is complete and visible.
+// result of this kernel while this kernel still runs.
 __device__ __forceinline__ void chain_wait() {
 #if defined(__CUDA_ARCH__)
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -97,7 +97,9 @@ long long bwmoe_launch_count(void);
  * `len`) and returns its length. */
 int bwmoe_last_error(char* buf, size_t len);
 
-/* Bytes of device workspace one forward of this shape needs (0 on a bad shape). */
+/* Bytes of device workspace one forward of this shape needs (0 on a bad shape).  Sizes are per batch, not growing with T
+ * throughout (split-K scratch is needed up to 64 slots only): a workspace that serves several batch sizes has the
+ * largest of their sizes, not the size of the largest batch. */
 size_t bwmoe_workspace_bytes(int T, int D, int H, int E, int K);
 
 /* Workspace size for bwmoe_moe_forward_host (0 on a bad shape). */
@@ -379,7 +381,8 @@ int bwmoe_gather_quant(const void* d_x, const int32_t* d_row_slot, const int32_t
  * Grouped gate+up FP8 GEMM with SwiGLU: h[m,:] = silu(gate) * up in bf16 with the
  * reference's bf16 rounding points, plus d_seg_amax_h[e] = max|h| per segment
  * (d_seg_amax_h must be zero on entry).  d_scratch needs bwmoe_gemm_scratch_bytes(M, D, H, E)
- * bytes (small batches split the K loop and sum fp32 partials from it in a fixed order).
+ * bytes (batches of up to 64 rows split the K loop and sum fp32 partials from it in a fixed order;
+ * beyond 64 rows the size falls to almost nothing, so a buffer that serves both is sized for min(M, 64)).
  * replaces: fused_gate_up_gemm, src/blackwell_moe/kernels/grouped_fp8_gateup.py:42-138,
  *           and F.silu(gate)*up, src/blackwell_moe/kernels/fp8_moe_v3.py:60.
  */
